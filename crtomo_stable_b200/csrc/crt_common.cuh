@@ -212,6 +212,74 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { cp_async_wait_group<0>(); }
 
+// FP64 tensor-core product D += A B (8 x 8 x 4).  Lane holds A[lane / 4]
+// [lane % 4], B[lane % 4][lane / 4] and D[lane / 4][2 (lane % 4) + 0, 1].  The
+// pipe forms each entry as the chain of fused multiply-adds over the four k in
+// order, so a sum taken in ascending order by fma() keeps its bits.
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+// An 8 x 8 accumulator tile of T and its update by KC entries of k (two
+// complex or four real ones per product).  A complex product is two chains,
+// real part [a.x, -a.y] . [b.x, b.y] and imaginary part [a.x, a.y] . [b.y,
+// b.x]: the order in which fma_acc / fms_acc take an entry's terms.  Lane:
+// row lane / 4, component or k lane % 4.
+template <typename T> struct MmaTile;
+template <> struct MmaTile<cd> {
+    static constexpr int KC = 2;
+    double x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+    struct A { double x, y; };   // the factors of the two chains
+    struct B { double n, s; };
+    // a / b: the entry of row (column) lane / 4 and k lane % 4 / 2
+    __device__ __forceinline__ static A lda(const cd* a)
+    {
+        const double v = reinterpret_cast<const double*>(a)[threadIdx.x & 1];
+        return A{(threadIdx.x & 1) ? -v : v, v};
+    }
+    __device__ __forceinline__ static A lda_neg(const cd* a)
+    {
+        const A v = lda(a);
+        return A{-v.x, -v.y};
+    }
+    __device__ __forceinline__ static B ldb(const cd* b)
+    {
+        const double* p = reinterpret_cast<const double*>(b);
+        return B{p[threadIdx.x & 1], p[(threadIdx.x & 1) ^ 1]};
+    }
+    __device__ __forceinline__ void mma(const A& a, const B& b)
+    {
+        dmma(x0, x1, a.x, b.n);
+        dmma(y0, y1, a.y, b.s);
+    }
+    __device__ __forceinline__ cd get(int c) const { return c ? cd{x1, y1} : cd{x0, y0}; }
+    __device__ __forceinline__ void set(int c, cd v)
+    {
+        if (c) x1 = v.x, y1 = v.y;
+        else x0 = v.x, y0 = v.y;
+    }
+    __device__ __forceinline__ static int kk() { return (threadIdx.x & 3) >> 1; }   // the lane's k of a product
+};
+template <> struct MmaTile<double> {
+    static constexpr int KC = 4;
+    double x0 = 0.0, x1 = 0.0;
+    using A = double;
+    using B = double;
+    __device__ __forceinline__ static A lda(const double* a) { return *a; }
+    __device__ __forceinline__ static A lda_neg(const double* a) { return -*a; }
+    __device__ __forceinline__ static B ldb(const double* b) { return *b; }
+    __device__ __forceinline__ void mma(A a, B b) { dmma(x0, x1, a, b); }
+    __device__ __forceinline__ double get(int c) const { return c ? x1 : x0; }
+    __device__ __forceinline__ void set(int c, double v)
+    {
+        if (c) x1 = v;
+        else x0 = v;
+    }
+    __device__ __forceinline__ static int kk() { return threadIdx.x & 3; }
+};
+
 // mbarrier and bulk-copy (TMA engine, untiled) helpers: one CTA, no cluster
 // multicast.  The wait gives up after a bounded number of polls and
 // reports failure instead of spinning for ever.

@@ -14,8 +14,8 @@
 //       by cp.async two blocks ahead; per block a 16-row triangle (half-warp
 //       per column, shuffle broadcasts) and an (mb x 16) x (16 x R) update
 //       in 4 x 4 register tiles;
-//   k_schur_gram    C = V^T [u^ | V^] per wavenumber (tiled GEMM that skips
-//       the rows where a column is still zero);
+//   k_schur_gram    C = V^T [u^ | V^] per wavenumber (tiled GEMM on the FP64
+//       tensor pipe that skips the rows where a column is still zero);
 //   k_schur_chol    per (k, l): S_l = A_GG(l) - V^T V^, right-looking
 //       blocked Cholesky (unconjugated, complex symmetric as
 //       src/chol.f90:44-78) with a 16-column panel in shared memory, the
@@ -651,16 +651,28 @@ __global__ void __launch_bounds__(512, 1) k_schur_sweep_pp(SchurArgs s, const T*
 
 // ---------------------------------------------------------------------------
 // C[k][c][g] = sum_i V^[i][g] X[i][c] over the rows where both columns can
-// be non-zero; tiles 64 (g) x 32 (c), 128 threads of 4 x 4.  The tiles of
-// the V^T V^ block above its diagonal are skipped (the Cholesky reads the
-// lower triangle).
-template <typename T>
-__global__ void __launch_bounds__(128) k_schur_gram(SchurArgs s, const T* __restrict__ X, T* C)
+// be non-zero, on the FP64 tensor pipe: tiles TG (g) x TC (c), warps of
+// (8 WG) x (8 WC), the rows staged GRAM_TI at a time, NS - 1 stages ahead.
+// Bound by the pipe and by the operands from L2 (1 KB per 4,096 multiply-adds
+// of a 32 x 32 tile); with the multiply-adds on the FP64 cores, 4 x 4 per
+// thread, their shared-memory operands bound it (60k triangles 14.3 -> 9.2 ms,
+// 20k cells 7.2 -> 4.0 ms, 12,960 cells real 0.72 -> 0.35 ms).
+// Every entry is summed over ascending rows.  The tiles of the V^T V^ block
+// above its diagonal are skipped (the Cholesky reads the lower triangle).
+// A row run of a column is padded by 32 bytes, so the four rows x 32 bytes
+// that a half-warp reads at once lie in different banks.
+constexpr int GRAM_TI = 16;
+template <typename T> struct RunPad { static constexpr int v = 32 / (int)sizeof(T); };
+
+template <typename T, int TG, int TC, int WG, int WC, int NS>
+__global__ void __launch_bounds__(TG / (8 * WG) * (TC / (8 * WC)) * 32)
+    k_schur_gram(SchurArgs s, const T* __restrict__ X, T* C)
 {
-    constexpr int TG = 64, TC = 32, TI = 16;
-    extern __shared__ __align__(16) unsigned char gram_dyn[];   // both stages of both tiles
-    auto As = reinterpret_cast<T(*)[TI][TG + 1]>(gram_dyn);                                  // [2][TI][TG + 1]
-    auto Bs = reinterpret_cast<T(*)[TI][TC + 1]>(gram_dyn + 2 * TI * (TG + 1) * sizeof(T));  // [2][TI][TC + 1]
+    constexpr int TI = GRAM_TI, ST = TI + RunPad<T>::v, NW = TC / (8 * WC), NT = TG / (8 * WG) * NW * 32;
+    using Tile = MmaTile<T>;
+    constexpr int KC = Tile::KC;
+    extern __shared__ __align__(16) unsigned char gram_dyn[];   // NS stages of both operands
+    T* buf0 = reinterpret_cast<T*>(gram_dyn);                   // [NS][TG + TC][ST]
     __shared__ int s_i0;
     // wavenumbers along x, so the long tiles (early first rows) of every
     // wavenumber start first
@@ -668,70 +680,69 @@ __global__ void __launch_bounds__(128) k_schur_gram(SchurArgs s, const T* __rest
     const int g0 = blockIdx.y * TG, c0 = blockIdx.z * TC;
     const int m = s.m, L = s.L, nI = s.nI, ncol = s.ncol;
     if (c0 >= L && c0 - L > g0 + TG - 1) return;
-    if (tid == 0) {
+    if (tid < 32) {
         int fg = nI, fc = nI;
-        for (int q = 0; q < TG && g0 + q < m; ++q) fg = min(fg, s.first[L + g0 + q]);
-        for (int q = 0; q < TC && c0 + q < ncol; ++q) fc = min(fc, s.first[c0 + q]);
-        s_i0 = max(fg, fc) / TI * TI;
+        for (int q = tid; q < TG && g0 + q < m; q += 32) fg = min(fg, s.first[L + g0 + q]);
+        for (int q = tid; q < TC && c0 + q < ncol; q += 32) fc = min(fc, s.first[c0 + q]);
+        const int f = max(__reduce_min_sync(0xffffffffu, fg), __reduce_min_sync(0xffffffffu, fc));
+        if (tid == 0) s_i0 = f / TI * TI;
     }
     __syncthreads();
-    const int ti = tid % 16, tc = tid / 16;
-    T acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[a][c] = Sc<T>::zero();
+    const int i0 = s_i0, nt = (nI - i0 + TI - 1) / TI;
+    const int lane = tid & 31, warp = tid >> 5, wg = warp / NW * 8 * WG, wc = warp % NW * 8 * WC;
+    Tile acc[WG][WC];
     const T* Xk = X + (size_t)k * ncol * nI;
-    // the tiles of rows [i0, i0 + TI) into buffer `buf` (cp.async, the
-    // next block's copies in flight while this one is multiplied)
-    auto stage = [&](int buf, int i0) {
-        for (int idx = tid; idx < TI * TG; idx += 128) {
-            const int gg = idx / TI, ii = idx % TI;
-            if (g0 + gg < m && i0 + ii < nI) cp_async_elem<T>(&As[buf][ii][gg], Xk + (size_t)(L + g0 + gg) * nI + i0 + ii);
-            else As[buf][ii][gg] = Sc<T>::zero();
+    // rows [i0 + t TI, + TI) of the tile's columns into stage t % NS
+    auto stage = [&](int t) {
+        T* dst = buf0 + (size_t)(t % NS) * (TG + TC) * ST;
+        const int r0 = i0 + t * TI;
+        for (int idx = tid; idx < TI * (TG + TC); idx += NT) {
+            const int q = idx / TI, ii = idx % TI;
+            const int c = q < TG ? (g0 + q < m ? L + g0 + q : -1) : (c0 + q - TG < ncol ? c0 + q - TG : -1);
+            T* d = dst + q * ST + ii;
+            if (c >= 0 && r0 + ii < nI) cp_async_elem<T>(d, Xk + (size_t)c * nI + r0 + ii);
+            else *d = Sc<T>::zero();
         }
-        for (int idx = tid; idx < TI * TC; idx += 128) {
-            const int cc = idx / TI, ii = idx % TI;
-            if (c0 + cc < ncol && i0 + ii < nI) cp_async_elem<T>(&Bs[buf][ii][cc], Xk + (size_t)(c0 + cc) * nI + i0 + ii);
-            else Bs[buf][ii][cc] = Sc<T>::zero();
-        }
-        cp_async_commit();
     };
-    int buf = 0;
-    if (s_i0 < nI) stage(0, s_i0);
-    for (int i0 = s_i0; i0 < nI; i0 += TI, buf ^= 1) {
-        if (i0 + TI < nI) {
-            stage(buf ^ 1, i0 + TI);   // its last readers finished before the trailing barrier
-            cp_async_wait_group<1>();
-        } else {
-            cp_async_wait_group<0>();
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int ii = 0; ii < TI; ++ii) {
-            T a4[4], b4[4];
-            // rows ti + 16 a, columns tc + 8 c: a warp reads consecutive words
-#pragma unroll
-            for (int a = 0; a < 4; ++a) a4[a] = As[buf][ii][ti + 16 * a];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b4[c] = Bs[buf][ii][tc + 8 * c];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) fma_acc(acc[a][c], a4[a], b4[c]);
-        }
-        __syncthreads();
+    for (int t = 0; t < NS - 1; ++t) {
+        if (t < nt) stage(t);
+        cp_async_commit();
     }
+    for (int t = 0; t < nt; ++t) {
+        cp_async_wait_group<NS - 2>();
+        __syncthreads();   // stage t has landed; the last readers of stage t - 1 are through
+        if (t + NS - 1 < nt) stage(t + NS - 1);
+        cp_async_commit();
+        const T* As = buf0 + (size_t)(t % NS) * (TG + TC) * ST;
+        const T* ap = As + (wg + (lane >> 2)) * ST + Tile::kk();
+        const T* bp = As + (TG + wc + (lane >> 2)) * ST + Tile::kk();
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int cc = c0 + tc + 8 * c;
-        if (cc >= ncol) continue;
+        for (int ii = 0; ii < TI; ii += KC) {
+            typename Tile::A a[WG];
+            typename Tile::B b[WC];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int g = g0 + ti + 16 * a;
-            if (g < m) C[((size_t)k * ncol + cc) * m + g] = acc[a][c];
+            for (int x = 0; x < WG; ++x) a[x] = Tile::lda(ap + x * 8 * ST + ii);
+#pragma unroll
+            for (int y = 0; y < WC; ++y) b[y] = Tile::ldb(bp + y * 8 * ST + ii);
+#pragma unroll
+            for (int x = 0; x < WG; ++x)
+#pragma unroll
+                for (int y = 0; y < WC; ++y) acc[x][y].mma(a[x], b[y]);
         }
     }
+    cp_async_wait_group<0>();
+#pragma unroll
+    for (int y = 0; y < WC; ++y)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int cc = c0 + wc + 8 * y + 2 * (lane & 3) + q;
+            if (cc >= ncol) continue;
+#pragma unroll
+            for (int x = 0; x < WG; ++x) {
+                const int g = g0 + wg + 8 * x + (lane >> 2);
+                if (g < m) C[((size_t)k * ncol + cc) * m + g] = acc[x][y].get(q);
+            }
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -1192,82 +1203,99 @@ __global__ void __launch_bounds__(SCHUR_IT_NT, MINB) k_schur_iter(SchurArgs s, B
 }
 
 // ---------------------------------------------------------------------------
-// z^_l = u^_l - V^ p_G: tiles of 64 interior rows x 32 electrodes; the
-// boundary columns in the order of their first row, so a tile stops at the
-// first column that is zero on all its rows.
+// z^_l = u^_l - V^ p_G on the FP64 tensor pipe (60k triangles 5.6 -> 5.0 ms
+// against 4 x 4 multiply-adds per thread): tiles of 64 interior rows x 32
+// electrodes (8 warps of 16 x 16); the boundary columns in the order of their
+// first row, so a tile stops at the first column that is zero on all its rows.
 template <typename T>
-__global__ void __launch_bounds__(128) k_schur_zrebuild(SchurArgs s, T* X, const T* __restrict__ xg)
+__global__ void __launch_bounds__(256) k_schur_zrebuild(SchurArgs s, T* X, const T* __restrict__ xg)
 {
-    constexpr int TI = 64, TL = 32, TG = 16;
-    extern __shared__ __align__(16) unsigned char zr_dyn[];   // both stages of both tiles
-    auto As = reinterpret_cast<T(*)[TG][TI + 1]>(zr_dyn);                                  // [2][TG][TI + 1]
-    auto Bs = reinterpret_cast<T(*)[TG][TL + 1]>(zr_dyn + 2 * TG * (TI + 1) * sizeof(T));  // [2][TG][TL + 1]
-    const int tid = threadIdx.x;
+    constexpr int TI = 64, TL = 32, TG = 16, NS = 3, NT = 256;
+    // [boundary column][row] and [electrode][boundary column] runs, padded so
+    // that what a half-warp reads at once (the columns of one product x four
+    // rows, four electrodes x the columns) lies in different banks
+    constexpr int SA = TI + 4, SB = TG + RunPad<T>::v;
+    using Tile = MmaTile<T>;
+    constexpr int KC = Tile::KC;
+    extern __shared__ __align__(16) unsigned char zr_dyn[];
+    T* buf0 = reinterpret_cast<T*>(zr_dyn);   // [NS][TG * SA + TL * SB]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // wavenumbers along x and the row blocks from the last: a late row block
     // meets the most boundary columns, so the longest tiles start first
     const int k = s.k0 + blockIdx.x, i0 = (gridDim.y - 1 - blockIdx.y) * TI, l0 = blockIdx.z * TL;
-    const int ti = tid % 16, tl = tid / 16;
     const int m = s.m, nI = s.nI, L = s.L;
     T* Xk = X + (size_t)k * s.ncol * nI;
-    T acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[a][c] = Sc<T>::zero();
-    // boundary columns [q0, q0 + TG) of both operands into buffer `buf`
-    // (cp.async, the next block's copies in flight during this one)
-    auto stage = [&](int buf, int q0) {
-        for (int idx = tid; idx < TG * TI; idx += 128) {
+    // boundary columns [TG t, TG t + TG) of both operands into stage t % NS
+    auto stage = [&](int t) {
+        T* As = buf0 + (size_t)(t % NS) * (TG * SA + TL * SB);
+        T* Bs = As + TG * SA;
+        for (int idx = tid; idx < TG * TI; idx += NT) {
             const int gg = idx / TI, ii = idx % TI;
-            const int g = q0 + gg < m ? s.gsort[q0 + gg] : -1;
-            if (g >= 0 && i0 + ii < nI) cp_async_elem<T>(&As[buf][gg][ii], Xk + (size_t)(L + g) * nI + i0 + ii);
-            else As[buf][gg][ii] = Sc<T>::zero();
+            const int g = TG * t + gg < m ? s.gsort[TG * t + gg] : -1;
+            if (g >= 0 && i0 + ii < nI) cp_async_elem<T>(As + gg * SA + ii, Xk + (size_t)(L + g) * nI + i0 + ii);
+            else As[gg * SA + ii] = Sc<T>::zero();
         }
-        for (int idx = tid; idx < TG * TL; idx += 128) {
+        for (int idx = tid; idx < TG * TL; idx += NT) {
             const int ll = idx / TG, gg = idx % TG;
-            const int g = q0 + gg < m ? s.gsort[q0 + gg] : -1;
-            if (g >= 0 && l0 + ll < L) cp_async_elem<T>(&Bs[buf][gg][ll], xg + ((size_t)k * L + l0 + ll) * m + g);
-            else Bs[buf][gg][ll] = Sc<T>::zero();
+            const int g = TG * t + gg < m ? s.gsort[TG * t + gg] : -1;
+            if (g >= 0 && l0 + ll < L) cp_async_elem<T>(Bs + ll * SB + gg, xg + ((size_t)k * L + l0 + ll) * m + g);
+            else Bs[ll * SB + gg] = Sc<T>::zero();
         }
-        cp_async_commit();
     };
     // the boundary columns in the order of their first rows: a block whose
     // first column starts below this tile ends the loop
-    auto live = [&](int q0) { return q0 < m && s.gfirst[q0] < i0 + TI; };
-    int buf = 0;
-    if (live(0)) stage(0, 0);
-    for (int q0 = 0; live(q0); q0 += TG, buf ^= 1) {
-        if (live(q0 + TG)) {
-            stage(buf ^ 1, q0 + TG);   // its last readers finished before the trailing barrier
-            cp_async_wait_group<1>();
-        } else {
-            cp_async_wait_group<0>();
+    auto live = [&](int t) { return TG * t < m && s.gfirst[TG * t] < i0 + TI; };
+    int nt = 0;
+    {   // the live blocks lead
+        int lo = 0, hi = (m + TG - 1) / TG;
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (live(mid)) lo = mid + 1;
+            else hi = mid;
         }
-        __syncthreads();
-#pragma unroll 4
-        for (int gg = 0; gg < TG; ++gg) {
-            T a4[4], b4[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) a4[a] = As[buf][gg][ti + 16 * a];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b4[c] = Bs[buf][gg][tl + 8 * c];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) fma_acc(acc[a][c], a4[a], b4[c]);
-        }
-        __syncthreads();
+        nt = lo;
     }
+    Tile acc[2][2];
+    const int wi = warp / 2 * 16, wl = warp % 2 * 16;
+    for (int t = 0; t < NS - 1; ++t) {
+        if (t < nt) stage(t);
+        cp_async_commit();
+    }
+    for (int t = 0; t < nt; ++t) {
+        cp_async_wait_group<NS - 2>();
+        __syncthreads();   // stage t has landed; the last readers of stage t - 1 are through
+        if (t + NS - 1 < nt) stage(t + NS - 1);
+        cp_async_commit();
+        const T* As = buf0 + (size_t)(t % NS) * (TG * SA + TL * SB);
+        const T* ap = As + Tile::kk() * SA + wi + (lane >> 2);
+        const T* bp = As + TG * SA + (wl + (lane >> 2)) * SB + Tile::kk();
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int l = l0 + tl + 8 * c;
-        if (l >= L) continue;
+        for (int gg = 0; gg < TG; gg += KC) {
+            typename Tile::A a[2];
+            typename Tile::B b[2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int i = i0 + ti + 16 * a;
-            if (i < nI) Xk[(size_t)l * nI + i] -= acc[a][c];
+            for (int x = 0; x < 2; ++x) a[x] = Tile::lda(ap + gg * SA + 8 * x);
+#pragma unroll
+            for (int y = 0; y < 2; ++y) b[y] = Tile::ldb(bp + 8 * y * SB + gg);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) acc[x][y].mma(a[x], b[y]);
         }
     }
+    cp_async_wait_group<0>();
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int l = l0 + wl + 8 * y + 2 * (lane & 3) + q;
+            if (l >= L) continue;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int i = i0 + wi + 8 * x + (lane >> 2);
+                if (i < nI) Xk[(size_t)l * nI + i] -= acc[x][y].get(q);
+            }
+        }
 }
 
 template <typename T>
@@ -1383,10 +1411,24 @@ void launch_wait_started(const int* started, int want, int* status, cudaStream_t
 template <typename T>
 void launch_schur_gram(const SchurArgs& s, const T* X, T* C, cudaStream_t st)
 {
-    dim3 grid(s.nk, (s.m + 63) / 64, (s.ncol + 31) / 32);
-    const int smem = 2 * 16 * (64 + 1 + 32 + 1) * (int)sizeof(T);   // the two stages of both tiles
-    cudaFuncSetAttribute(k_schur_gram<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_schur_gram<T><<<grid, 128, smem, st>>>(s, X, C);
+    auto go = [&](auto kern, int TG, int TC, int nt, int ns) {
+        const int smem = ns * (TG + TC) * (GRAM_TI + RunPad<T>::v) * (int)sizeof(T);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        kern<<<dim3(s.nk, (s.m + TG - 1) / TG, (s.ncol + TC - 1) / TC), nt, smem, st>>>(s, X, C);
+    };
+    // 32 x 32 tiles, or 32 x 16 where there would be fewer than five per SM
+    // (8,000 triangles and 48 electrodes, 12 wavenumbers: 0.34 against 0.45
+    // ms; 60k triangles: 9.7 against 9.2 ms, the other way).  64-wide tiles
+    // lose on every size (60k triangles: 12.5 ms at 64 x 64, 10.8 at 64 x 32):
+    // a tile runs from the earliest row of its columns, and its serial sum
+    // over the rows is the longest CTA's time.
+    int nsm = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if ((long long)s.nk * ((s.m + 31) / 32) * ((s.ncol + 31) / 32) >= 5 * nsm)
+        go(k_schur_gram<T, 32, 32, 2, 2, 4>, 32, 32, 128, 4);
+    else
+        go(k_schur_gram<T, 32, 16, 2, 1, 4>, 32, 16, 128, 4);
 }
 
 template <typename T>
@@ -1478,9 +1520,10 @@ template <typename T>
 void launch_schur_zrebuild(const SchurArgs& s, T* X, const T* xg, cudaStream_t st)
 {
     dim3 grid(s.nk, (s.nI + 63) / 64, (s.L + 31) / 32);
-    const int smem = 2 * 16 * (64 + 1 + 32 + 1) * (int)sizeof(T);   // the two stages of both tiles
+    constexpr int smem = 3 * (16 * (64 + 4) + 32 * (16 + RunPad<T>::v)) *
+                         (int)sizeof(T);   // three stages of both operands
     cudaFuncSetAttribute(k_schur_zrebuild<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_schur_zrebuild<T><<<grid, 128, smem, st>>>(s, X, xg);
+    k_schur_zrebuild<T><<<grid, 256, smem, st>>>(s, X, xg);
 }
 
 template <typename T>

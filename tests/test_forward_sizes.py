@@ -1,0 +1,43 @@
+"""Forward potentials at the sizes where the kernels' tiles,
+panels and row blocks have remainders, against the oracle."""
+import numpy as np
+import pytest
+
+from crtomo_stable_b200 import synth
+
+RTOL = 1e-10       # of the largest potential / voltage: the other parity tests' bound
+
+
+def survey(nx, nz, nel, tri, seed=3):
+    rng = np.random.default_rng(seed)
+    xs = np.arange(nx + 1, dtype=np.float64) - (nx - nel) // 2
+    mesh = synth.structured_mesh(xs, synth.graded_depths(nz, 0.4, 1.0 + 2.0 / nz), triangles=tri)
+    enr = synth.surface_electrodes(mesh, xs, np.arange(nel, dtype=np.float64), nz)
+    configs = synth.dipole_dipole(nel, (1, 2), 6) if nel >= 4 else [(1, 0, 2, 0)]
+    strnr, vnr = synth.encode(configs)
+    rho = np.exp(rng.uniform(np.log(10.0), np.log(1000.0), mesh.elanz))
+    return mesh, enr, strnr, vnr, synth.sigma_from(rho, -rng.uniform(1.0, 30.0, mesh.elanz))
+
+
+# (cells, cells, electrodes, triangles): half-bandwidths 4 to 131, boundary
+# sets of 9 to 350 nodes, interiors of a single panel up to 6,400 rows
+SIZES = [(4, 2, 2, True), (6, 3, 4, False), (9, 7, 5, True), (33, 8, 17, False), (20, 31, 12, True),
+         (40, 15, 33, True), (24, 64, 10, False), (28, 130, 9, True), (180, 36, 96, True)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ldc", [False, True])
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(str(int(v)) for v in s))
+def test_forward_potentials(size, ldc):
+    from crtomo_stable_b200.lib import FORWARD_SCHUR, Context
+    from oracle.oracle import OracleProblem
+    mesh, enr, strnr, vnr, sigma = survey(*size)
+    ctx = Context(mesh, enr, strnr, vnr)
+    op = OracleProblem(mesh, enr, strnr, vnr, kwn=ctx.kwn, kwnwi=ctx.kwnwi)
+    kp_o = op.forward(sigma, ldc=ldc, nthreads=8)
+    volt_o, _ = op.bvolti(op.rtrafo(kp_o))
+    volt, _, kp = ctx.forward(sigma, ldc=ldc, want_kpot=True)
+    assert ctx.forward_info()[0] == FORWARD_SCHUR
+    assert np.abs(kp - kp_o).max() <= RTOL * np.abs(kp_o).max()
+    assert np.abs(volt - volt_o).max() <= RTOL * np.abs(volt_o).max()
+    ctx.close()
