@@ -1121,9 +1121,13 @@ int run_forward_schur(crt_ctx* ctx)
     mk.e0 = tev_rec(ctx);
     const bool blk = band_blk_fits<T>(H.mbI);
     int pb = 0;
+    const char* fv = std::getenv("CRT_B200_FACTOR");
+    // the window in registers (CRT_B200_FACTOR=blk, or a panel width fixed by
+    // CRT_B200_PANEL: the panel-blocked kernel)
+    const bool mma = band_mma_fits<T>(H.mbI) && !(fv && std::strcmp(fv, "blk") == 0) && !std::getenv("CRT_B200_PANEL");
     if (blk) {
-        pb = band_panel<T>(AI, !ctx->capture, ctx->st);
-        ctx->panel = pb & BAND_PANEL_MASK;
+        if (!mma) pb = band_panel<T>(AI, !ctx->capture, ctx->st);
+        ctx->panel = mma ? 8 : pb & BAND_PANEL_MASK;
         launch_band_prep<T>(AI, ctx->st);   // the scaling factors for the right-hand sides
     }
     CK(cudaMemsetAsync(X, 0, sizeof(T) * (size_t)K * ncol * nI, ctx->st));
@@ -1150,7 +1154,8 @@ int run_forward_schur(crt_ctx* ctx)
             AI.started = ctx->d_fprog + K;
             CK(cudaEventRecord(ctx->ovl_ev[0], ctx->st));
         }
-        launch_band_factor_blk<T>(AI, pb, ctx->st);
+        if (mma) launch_band_factor_mma<T>(AI, ctx->st);
+        else launch_band_factor_blk<T>(AI, pb, ctx->st);
     } else {
         launch_band_factor<T>(AI, ctx->st);   // forms fak as it goes
         launch_schur_rhs<T>(S, Af, ctx->d_sfak, X, cval, ctx->st);

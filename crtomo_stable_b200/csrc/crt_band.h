@@ -134,6 +134,10 @@ template <typename T> bool launch_band_factor_blk(const BandArgs<T>& a, int cfg,
 // up to two waves of a's systems when may_tune (it prepares and factors
 // them, so the caller prepares them again), else returns panel 8.
 template <typename T> int band_panel(const BandArgs<T>& a, bool may_tune, cudaStream_t st);
+// Factorisation of few systems without right-hand sides (at most one per SM)
+// with the window in registers (crt_band_mma.cu); half-bandwidths up to 128.
+template <typename T> bool band_mma_fits(int mb);
+template <typename T> void launch_band_factor_mma(const BandArgs<T>& a, cudaStream_t st);
 // Whether the panel-blocked window fits in shared memory for half-bandwidth mb.
 template <typename T> bool band_blk_fits(int mb);
 // Preparation pass of the panel-blocked factor: assembled, Dirichlet-edited

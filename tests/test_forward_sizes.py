@@ -22,7 +22,8 @@ def survey(nx, nz, nel, tri, seed=3):
 # (cells, cells, electrodes, triangles): half-bandwidths 4 to 131, boundary
 # sets of 9 to 350 nodes, interiors of a single panel up to 6,400 rows
 SIZES = [(4, 2, 2, True), (6, 3, 4, False), (9, 7, 5, True), (33, 8, 17, False), (20, 31, 12, True),
-         (40, 15, 33, True), (24, 64, 10, False), (28, 130, 9, True), (180, 36, 96, True)]
+         (40, 15, 33, True), (24, 64, 10, False), (20, 80, 9, True), (16, 127, 7, True), (28, 130, 9, True),
+         (180, 36, 96, True)]
 
 
 @pytest.mark.gpu
@@ -41,3 +42,24 @@ def test_forward_potentials(size, ldc):
     assert np.abs(kp - kp_o).max() <= RTOL * np.abs(kp_o).max()
     assert np.abs(volt - volt_o).max() <= RTOL * np.abs(volt_o).max()
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,nz,panel", [(12, 2, 4), (14, 7, 4), (14, 16, 4), (15, 17, 4), (14, 25, 4), (14, 33, 4),
+                                         (13, 41, 4), (13, 57, 4), (12, 66, 4), (12, 75, 4), (12, 77, 8), (12, 88, 8),
+                                         (12, 90, 4), (12, 100, 4), (12, 106, 8), (12, 112, 8), (12, 127, 8)])
+def test_factor_in_registers_is_the_panel_blocked_factor(nx, nz, panel, monkeypatch):
+    """The interior factor with its window in registers against the
+    panel-blocked kernel at the panel width whose order of products it keeps:
+    the same potentials bit for bit, complex and real."""
+    from crtomo_stable_b200.lib import Context
+    mesh, enr, strnr, vnr, sigma = survey(nx, nz, 5, nz % 2 == 0)
+    out = []
+    for blocked in (False, True):
+        if blocked:
+            monkeypatch.setenv("CRT_B200_PANEL", str(panel))
+        ctx = Context(mesh, enr, strnr, vnr)
+        out.append([ctx.forward(sigma, ldc=ldc, want_kpot=True)[2] for ldc in (False, True)])
+        ctx.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
