@@ -110,6 +110,7 @@ struct crt_ctx {
     CGState* d_live = nullptr;   // a never-done CG state for preconditioner applications outside the CG
     double* d_vred = nullptr;    // partial sums of the CG head and tail
     cd* d_sfac = nullptr;        // per-reading factors of the Gram-form Jacobian
+    double* d_colsum = nullptr;  // sums over the Jacobian's columns and readings (lambda_0, coverage), kept
     // the forward sweep concurrent with the interior factor: the factor's
     // progress per wavenumber and its count of started CTAs, the stream and
     // the fork / join events
@@ -418,7 +419,7 @@ extern "C" void crt_destroy(crt_ctx* ctx)
                     ctx->d_fakws, ctx->d_scratch, ctx->d_sens, ctx->d_part_sens, ctx->d_strom, ctx->d_smatm,
                     ctx->d_nachbar, ctx->d_dat, ctx->d_wd, ctx->d_cgfac, ctx->d_cgres, ctx->d_bdpar,
                     ctx->d_rhs, ctx->d_p, ctx->d_r, ctx->d_bvec, ctx->d_dpar, ctx->d_ap, ctx->d_cgpart,
-                    ctx->d_par, ctx->d_par_backup, ctx->d_cgst, ctx->d_z, ctx->d_rold, ctx->d_zb, ctx->d_live, ctx->d_cgl, ctx->d_omega, ctx->d_cgf, ctx->d_vred, ctx->d_sfac, ctx->d_fprog,
+                    ctx->d_par, ctx->d_par_backup, ctx->d_cgst, ctx->d_z, ctx->d_rold, ctx->d_zb, ctx->d_live, ctx->d_cgl, ctx->d_omega, ctx->d_cgf, ctx->d_vred, ctx->d_sfac, ctx->d_colsum, ctx->d_fprog,
                     ctx->d_dc_rows, ctx->d_dc_ptr, ctx->d_dc_ent, ctx->d_dc_node, ctx->d_bdir};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1755,8 +1756,9 @@ int update_device(crt_ctx* ctx, const crt_cg_params* prm, const cd* d_sigmaa, in
     ctx->cg_form = use_block ? (use_gnn ? CRT_PRECOND_BLOCK_GNN : CRT_PRECOND_BLOCK)
                              : (use_gnn ? CRT_PRECOND_GNN : CRT_PRECOND_JACOBI);
     if (int e = setup_cg_fused(ctx, &a)) return e;
+    a.turn = !a.pc;
     launch_cg_init(a, ctx->st);
-    ctx->launches += 1;
+    ctx->launches += a.turn ? 3 : 1;
     CK(cudaEventRecord(ctx->ev[1], ctx->st));
     if (int e = kernel_check(ctx, "cg setup")) return e;
     // iterate in batches; the device-side stop flag makes surplus launches no-ops
@@ -1767,7 +1769,7 @@ int update_device(crt_ctx* ctx, const crt_cg_params* prm, const cd* d_sigmaa, in
         int it = std::min(batch, prm->ncgmax - done_iters);
         launch_cg_iterations(a, it, use_block ? &ctx->spc : nullptr, use_gnn ? &ctx->gnn : nullptr, ctx->d_zb,
                              ctx->st);
-        ctx->launches += ((a.fused ? 5 : 7) + (a.pc ? 1 : 0) + (use_block ? 2 : 0) + (use_gnn ? 7 : 0)) * it;
+        ctx->launches += ((a.fused ? 5 : 7) - (a.turn ? 3 : 0) + (a.pc ? 1 : 0) + (use_block ? 2 : 0) + (use_gnn ? 7 : 0)) * it;
         done_iters += it;
         CK(cudaMemcpyAsync(&hs, ctx->d_cgst, sizeof(CGState), cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
@@ -1820,13 +1822,31 @@ template <> __device__ __forceinline__ cd jval<cf>(const cf* J, size_t idx)
 template <> __device__ __forceinline__ cd jval<double>(const double* J, size_t idx) { return cd{J[idx], 0.0}; }
 template <> __device__ __forceinline__ cd jval<float>(const float* J, size_t idx) { return cd{(double)J[idx], 0.0}; }
 
+// Row sums over BLAM0_SPLIT ranges of the cells (grid.y; a thread per reading
+// and range, 8 loads in flight), then the ranges' sums in order into s[0 .. N).
+// One range per reading left 3 CTAs on the GPU: 773 us for 735 readings of
+// 8,000 cells.
+constexpr int BLAM0_SPLIT = 64;
+
 template <typename S>
-__global__ void k_blam0_rowsum(const S* __restrict__ J, int N, int M, int re_part, cd* s)
+__global__ void k_blam0_rowsum(const S* __restrict__ J, int N, int M, cd* part)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const int per = (M + gridDim.y - 1) / gridDim.y, j0 = blockIdx.y * per, j1 = min(M, j0 + per);
+    cd acc{0.0, 0.0};
+#pragma unroll 8
+    for (int j = j0; j < j1; ++j) acc += jval<S>(J, (size_t)j * N + i);
+    part[(size_t)blockIdx.y * N + i] = acc;
+}
+
+__global__ void k_blam0_rowadd(const cd* __restrict__ part, int N, int re_part, cd* s)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     cd acc{0.0, 0.0};
-    for (int j = 0; j < M; ++j) acc += jval<S>(J, (size_t)j * N + i);
+#pragma unroll 16
+    for (int q = 0; q < BLAM0_SPLIT; ++q) acc += part[(size_t)q * N + i];
     if (re_part) acc.y = 0.0;
     s[i] = acc;
 }
@@ -1869,11 +1889,22 @@ __global__ void k_coverage_col(const S* __restrict__ J, int N, int M, int re_par
     if (lane == 0) csens[j] = acc;
 }
 
+// Readings' sums (blam0) or weights (coverage), then a double per cell: one
+// buffer, allocated at the first call (an allocation and a release per call
+// cost up to milliseconds)
+int ensure_colsum(crt_ctx* ctx)
+{
+    if (ctx->d_colsum) return CRT_OK;
+    return dalloc(ctx, &ctx->d_colsum, 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT) + (size_t)ctx->E) ? CRT_OK : CRT_ERR_CUDA;
+}
+
 template <typename S>
 void blam0_launch(const crt_ctx* ctx, int re_part, cd* s, double* jtj)
 {
     const S* J = static_cast<const S*>(ctx->d_sens);
-    k_blam0_rowsum<S><<<(ctx->N + 255) / 256, 256, 0, ctx->st>>>(J, ctx->N, ctx->E, re_part, s);
+    cd* part = s + ctx->N;
+    k_blam0_rowsum<S><<<dim3((ctx->N + 127) / 128, BLAM0_SPLIT), 128, 0, ctx->st>>>(J, ctx->N, ctx->E, part);
+    k_blam0_rowadd<<<(ctx->N + 127) / 128, 128, 0, ctx->st>>>(part, ctx->N, re_part, s);
     k_blam0_col<S><<<(ctx->E * 32 + 255) / 256, 256, 0, ctx->st>>>(J, ctx->N, ctx->E, re_part, ctx->d_wd, s, jtj);
 }
 
@@ -1887,13 +1918,9 @@ extern "C" int32_t crt_blam0(crt_ctx* ctx, int32_t ldc, int32_t lfpi, double alf
     if ((ldc != 0) != (ctx->sens_real != 0))
         return set_err(ctx, CRT_ERR_ARG, "crt_blam0: ldc does not match the stored Jacobian");
     CK(cudaSetDevice(ctx->device));
-    cd* s = nullptr;
-    double* jtj = nullptr;
-    CK(cudaMalloc((void**)&s, sizeof(cd) * (size_t)ctx->N));
-    if (cudaMalloc((void**)&jtj, sizeof(double) * (size_t)ctx->E) != cudaSuccess) {
-        cudaFree(s);
-        return set_err(ctx, CRT_ERR_CUDA, "cudaMalloc of the blam0 sums");
-    }
+    if (int e = ensure_colsum(ctx)) return e;
+    cd* s = reinterpret_cast<cd*>(ctx->d_colsum);
+    double* jtj = ctx->d_colsum + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
     const bool f32 = ctx->prec == CRT_PREC_MIXED;
     if (ldc) {
         if (f32) blam0_launch<float>(ctx, 0, s, jtj);
@@ -1902,14 +1929,12 @@ extern "C" int32_t crt_blam0(crt_ctx* ctx, int32_t ldc, int32_t lfpi, double alf
         if (f32) blam0_launch<cf>(ctx, lfpi != 0, s, jtj);
         else blam0_launch<cd>(ctx, lfpi != 0, s, jtj);
     }
-    ctx->launches += 2;
+    ctx->launches += 3;
     std::vector<double> h(ctx->E);
     int e = kernel_check(ctx, "blam0");
     if (!e && cudaMemcpyAsync(h.data(), jtj, sizeof(double) * ctx->E, cudaMemcpyDeviceToHost, ctx->st) != cudaSuccess)
         e = set_err(ctx, CRT_ERR_CUDA, "blam0 copy");
     if (!e && cudaStreamSynchronize(ctx->st) != cudaSuccess) e = set_err(ctx, CRT_ERR_CUDA, "blam0 sync");
-    cudaFree(s);
-    cudaFree(jtj);
     if (e) return e;
     double tot = 0.0;
     for (double v : h) tot += v;
@@ -1923,19 +1948,9 @@ extern "C" int32_t crt_coverage(crt_ctx* ctx, int32_t part, const double* weight
     if (!ctx->have_sens || !ctx->d_sens) return set_err(ctx, CRT_ERR_ARG, "crt_coverage before crt_jacobian");
     if (!weight && !ctx->d_wd) return set_err(ctx, CRT_ERR_ARG, "crt_coverage without weights before crt_set_data");
     CK(cudaSetDevice(ctx->device));
-    double *w = nullptr, *cs = nullptr;
-    CK(cudaMalloc((void**)&cs, sizeof(double) * (size_t)ctx->E));
-    if (weight) {
-        if (cudaMalloc((void**)&w, sizeof(double) * (size_t)ctx->N) != cudaSuccess) {
-            cudaFree(cs);
-            return set_err(ctx, CRT_ERR_CUDA, "cudaMalloc of the coverage weights");
-        }
-        if (cudaMemcpyAsync(w, weight, sizeof(double) * ctx->N, cudaMemcpyHostToDevice, ctx->st) != cudaSuccess) {
-            cudaFree(cs);
-            cudaFree(w);
-            return set_err(ctx, CRT_ERR_CUDA, "coverage weights copy");
-        }
-    }
+    if (int e = ensure_colsum(ctx)) return e;
+    double *w = ctx->d_colsum, *cs = ctx->d_colsum + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
+    if (weight) CK(cudaMemcpyAsync(w, weight, sizeof(double) * ctx->N, cudaMemcpyHostToDevice, ctx->st));
     const double* wd = weight ? w : ctx->d_wd;
     const int sq = weight ? 0 : 1, g = (ctx->E * 32 + 255) / 256;
     const bool f32 = ctx->prec == CRT_PREC_MIXED;
@@ -1951,8 +1966,6 @@ extern "C" int32_t crt_coverage(crt_ctx* ctx, int32_t part, const double* weight
     if (!e && cudaMemcpyAsync(csens, cs, sizeof(double) * ctx->E, cudaMemcpyDeviceToHost, ctx->st) != cudaSuccess)
         e = set_err(ctx, CRT_ERR_CUDA, "coverage copy");
     if (!e && cudaStreamSynchronize(ctx->st) != cudaSuccess) e = set_err(ctx, CRT_ERR_CUDA, "coverage sync");
-    cudaFree(cs);
-    if (w) cudaFree(w);
     return e;
 }
 
@@ -2137,7 +2150,7 @@ extern "C" int32_t crt_update_lambdas(crt_ctx* ctx, const crt_cg_params* prm, in
     }
     L.a.pc = use_block ? 1 : 0;
     launch_cgl_init(L, ctx->st);
-    ctx->launches += 1;
+    ctx->launches += use_block ? 1 : 2;
     CK(cudaEventRecord(ctx->ev[1], ctx->st));
     if (int e = kernel_check(ctx, "lambda-batch cg setup")) return e;
     std::vector<CGState> hs(nl);

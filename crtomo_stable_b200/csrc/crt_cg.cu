@@ -30,6 +30,19 @@ namespace {
 
 constexpr int VEC_NT = 1024;
 
+// An iteration is a chain of short kernels.  They are launched with
+// programmatic stream serialisation: each lets the next one's CTAs start as
+// soon as its own have all begun, and every thread waits here until the
+// kernel before has completed and its writes are visible, before it reads
+// anything (a kernel that returned without waiting would let a later one run
+// beside an earlier).  Between two kernels 2.4 us pass without it (9,600 cells,
+// 1,224 readings: 17 of an iteration's 109 us).
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 // J(i, e) as an FP64 complex value: JP selects the storage precision,
 // JM the Jacobian form (complex, real sensdc, real part of complex).
 template <int JP, int JM>
@@ -414,6 +427,7 @@ template <int JP, int JM>
 __global__ void __launch_bounds__(JV_NT) k_cg_jv(CGArgs A)
 {
     __shared__ cd pcs[JV_CHUNK];
+    chain_wait();
     if (A.st->done) return;
     const int i = blockIdx.x * JV_NT + threadIdx.x;
     const bool valid = i < A.N;
@@ -440,15 +454,31 @@ __global__ void __launch_bounds__(JV_NT) k_cg_jv(CGArgs A)
     if (valid) A.part[(size_t)split * A.N + i] = acc;
 }
 
+// Reading i's partial sums, added in order, 16 loads in flight (one after the
+// other they took 8 us).
+__device__ __forceinline__ cd sum_parts(const CGArgs& A, int i)
+{
+    cd acc{0.0, 0.0};
+    for (int s0 = 0; s0 < A.nsplit; s0 += 16) {
+        cd v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            if (s0 + q < A.nsplit) v[q] = A.part[(size_t)(s0 + q) * A.N + i];
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            if (s0 + q < A.nsplit) acc += v[q];
+    }
+    return acc;
+}
+
 // ap = sum of the partial sums; what the transposed product needs is w o ap.
 __global__ void k_cg_jv_reduce(CGArgs A)
 {
+    chain_wait();
     if (A.st->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.N) return;
-    cd acc{0.0, 0.0};
-    for (int s = 0; s < A.nsplit; ++s) acc += A.part[(size_t)s * A.N + i];
-    A.ap[i] = acc * A.wd[i];
+    A.ap[i] = sum_parts(A, i) * A.wd[i];
 }
 
 // b_e = (sum_i conj(J_ie) (w o ap)_i + lam (R (cgfac o p))_e) * cgfac_e,
@@ -465,6 +495,7 @@ __global__ void __launch_bounds__(JH_NT) k_cg_jhv(CGArgs A)
 {
     using RT = typename JRaw<JP, JM>::T;
     __shared__ __align__(16) cd s_ap[2][JH_CHUNK];
+    chain_wait();
     if (A.st->done) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ebase = (blockIdx.x * (JH_NT / 32) + warp) * NC;
@@ -820,6 +851,7 @@ __device__ bool vs_gather(const CGArgs& A, const double (&q)[n], double (&tot)[n
 
 __global__ void __launch_bounds__(32) k_cg_head_sums(CGArgs A)
 {
+    chain_wait();
     if (A.st->done) return;
     double v = 0.0;
     for (int e = blockIdx.x * 32 + threadIdx.x; e < A.M; e += VEC_NT) v += cabs2(A.r[e]);
@@ -830,6 +862,7 @@ __global__ void __launch_bounds__(32) k_cg_head_sums(CGArgs A)
 
 __global__ void __launch_bounds__(VS_UPD_NT) k_cg_head_update(CGArgs A)
 {
+    chain_wait();
     const CGState* st = A.st;
     if (st->done) return;
     const int e = blockIdx.x * VS_UPD_NT + threadIdx.x;
@@ -840,6 +873,7 @@ __global__ void __launch_bounds__(VS_UPD_NT) k_cg_head_update(CGArgs A)
 
 __global__ void __launch_bounds__(32) k_cg_head_pc_sums(CGArgs A)
 {
+    chain_wait();
     CGState* st = A.st;
     if (st->done) return;
     const bool guard = A.pc_gnn != 0;
@@ -870,6 +904,7 @@ __global__ void __launch_bounds__(32) k_cg_head_pc_sums(CGArgs A)
 
 __global__ void __launch_bounds__(VS_UPD_NT) k_cg_head_pc_update(CGArgs A)
 {
+    chain_wait();
     const CGState* st = A.st;
     if (st->done) return;
     const int e = blockIdx.x * VS_UPD_NT + threadIdx.x;
@@ -883,6 +918,7 @@ __global__ void __launch_bounds__(VS_UPD_NT) k_cg_head_pc_update(CGArgs A)
 
 __global__ void __launch_bounds__(32) k_cg_tail_sums(CGArgs A)
 {
+    chain_wait();
     CGState* st = A.st;
     if (st->done) return;
     double v = 0.0;
@@ -904,6 +940,7 @@ __global__ void __launch_bounds__(32) k_cg_tail_sums(CGArgs A)
 __global__ void __launch_bounds__(VS_UPD_NT) k_cg_tail_update(CGArgs A)
 {
     __shared__ int s_go;
+    chain_wait();
     CGState* st = A.st;
     if (threadIdx.x == 0) s_go = st->pending;
     __syncthreads();
@@ -919,6 +956,94 @@ __global__ void __launch_bounds__(VS_UPD_NT) k_cg_tail_update(CGArgs A)
         st->ucnt = 0;
         st->pending = 0;
     }
+}
+
+// Tail of one iteration and head of the next, Jacobi form, by one cluster of
+// 8 CTAs (VEC_NT threads, thread g taking the elements g + VEC_NT k and the
+// sums' order of the one-CTA form): the two dot products cross the cluster
+// through its shared memory, and the vectors pass twice.  Against two sums
+// and two updates across the grid 14.6 us of kernels and three launches less
+// per iteration (9,600 cells).
+constexpr int TURN_CTAS = 8, TURN_NT = VEC_NT / TURN_CTAS, TURN_UNROLL = 4;
+
+// the total of v over the cluster, in every thread; `slot` has a double per
+// warp of the cluster
+__device__ __forceinline__ double cluster_total(double v, double* slot, int gwarp)
+{
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) < TURN_CTAS) {
+        // lane q writes the warp's sum into CTA q's shared memory
+        v = __shfl_sync(0xffu, v, 0);
+        unsigned dst;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                     : "=r"(dst)
+                     : "r"((unsigned)__cvta_generic_to_shared(slot + gwarp)), "r"(threadIdx.x & 31));
+        asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(dst), "d"(v) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    return warp_allsum(slot[threadIdx.x & 31]);
+}
+
+__device__ void cg_turn_body(const CGArgs& A)
+{
+    __shared__ double slot[2][VEC_NT / 32];
+    CGState* st = A.st;
+    if (st->done) return;   // the same for the whole cluster: it is written after both sums
+    const int g = (blockIdx.x % TURN_CTAS) * TURN_NT + threadIdx.x;
+    const double num = st->num, dr_k = st->dr, dr0 = st->dr0;
+    const int k = st->k;
+    double v = 0.0;
+    for (int e0 = g; e0 < A.M; e0 += TURN_UNROLL * VEC_NT) {
+        cd pp[TURN_UNROLL], bb[TURN_UNROLL];
+#pragma unroll
+        for (int q = 0; q < TURN_UNROLL; ++q)
+            if (e0 + q * VEC_NT < A.M) pp[q] = A.p[e0 + q * VEC_NT], bb[q] = A.bvec[e0 + q * VEC_NT];
+#pragma unroll
+        for (int q = 0; q < TURN_UNROLL; ++q)
+            if (e0 + q * VEC_NT < A.M) v += pp[q].x * bb[q].x + pp[q].y * bb[q].y;
+    }
+    const double alpha = num / cluster_total(v, slot[0], g >> 5);
+    v = 0.0;
+    for (int e0 = g; e0 < A.M; e0 += TURN_UNROLL * VEC_NT) {
+        cd pp[TURN_UNROLL], bb[TURN_UNROLL], rr[TURN_UNROLL], dd[TURN_UNROLL];
+#pragma unroll
+        for (int q = 0; q < TURN_UNROLL; ++q) {
+            const int e = e0 + q * VEC_NT;
+            if (e < A.M) pp[q] = A.p[e], bb[q] = A.bvec[e], rr[q] = A.r[e], dd[q] = A.dpar[e];
+        }
+#pragma unroll
+        for (int q = 0; q < TURN_UNROLL; ++q) {
+            const int e = e0 + q * VEC_NT;
+            if (e >= A.M) continue;
+            A.dpar[e] = dd[q] + pp[q] * alpha;
+            rr[q] = rr[q] - bb[q] * alpha;
+            A.r[e] = rr[q];
+            v += cabs2(rr[q]);
+        }
+    }
+    const double dr = cluster_total(v, slot[1], g >> 5);
+    const bool go = k + 1 <= A.ncgmax && !(dr <= dr0);
+    const double beta = dr / dr_k;
+    if (go)
+        for (int e0 = g; e0 < A.M; e0 += TURN_UNROLL * VEC_NT) {
+            cd pp[TURN_UNROLL], rr[TURN_UNROLL];
+#pragma unroll
+            for (int q = 0; q < TURN_UNROLL; ++q)
+                if (e0 + q * VEC_NT < A.M) pp[q] = A.p[e0 + q * VEC_NT], rr[q] = A.r[e0 + q * VEC_NT];
+#pragma unroll
+            for (int q = 0; q < TURN_UNROLL; ++q)
+                if (e0 + q * VEC_NT < A.M) A.p[e0 + q * VEC_NT] = rr[q] + pp[q] * beta;
+        }
+    if (g == 0) {
+        tail_decide(A, alpha);
+        if (!st->done) head_decide(A, dr);
+    }
+}
+
+__global__ void __cluster_dims__(TURN_CTAS, 1, 1) __launch_bounds__(TURN_NT) k_cg_turn(CGArgs A)
+{
+    chain_wait();
+    cg_turn_body(A);
 }
 
 __device__ void cg_finish_body(const CGArgs& A, int lfpi, double step, const cd* par_in, cd* par,
@@ -1019,6 +1144,11 @@ __global__ void __launch_bounds__(VEC_NT) k_cgl_init(CGLArgs L) { cg_init_body(c
 __global__ void __launch_bounds__(VEC_NT) k_cgl_begin(CGLArgs L) { cg_begin_body(cgl_cand(L, blockIdx.x)); }
 __global__ void __launch_bounds__(VEC_NT) k_cgl_begin_pc(CGLArgs L) { cg_begin_pc_body(cgl_cand(L, blockIdx.x)); }
 __global__ void __launch_bounds__(VEC_NT) k_cgl_end(CGLArgs L) { cg_end_body(cgl_cand(L, blockIdx.x)); }
+__global__ void __cluster_dims__(TURN_CTAS, 1, 1) __launch_bounds__(TURN_NT) k_cgl_turn(CGLArgs L)
+{
+    chain_wait();
+    cg_turn_body(cgl_cand(L, blockIdx.x / TURN_CTAS));
+}
 __global__ void __launch_bounds__(VEC_NT) k_cgl_finish(CGLArgs L, int lfpi, double step, const cd* par_in,
                                                        cd* par_out, double* bdpar)
 {
@@ -1032,6 +1162,7 @@ template <int JP, int JM, int NL>
 __global__ void __launch_bounds__(JV_NT) k_cgl_jv(CGLArgs L)
 {
     __shared__ cd pcs[NL][JV_CHUNK];
+    chain_wait();
     if (cgl_all_done(L)) return;
     const CGArgs& A = L.a;
     const size_t M = (size_t)A.M;
@@ -1080,13 +1211,12 @@ __global__ void __launch_bounds__(JV_NT) k_cgl_jv(CGLArgs L)
 // k_cg_jv_reduce per candidate (grid.y = candidate).
 __global__ void k_cgl_jv_reduce(CGLArgs L)
 {
+    chain_wait();
     const CGArgs A = cgl_cand(L, blockIdx.y);
     if (A.st->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.N) return;
-    cd acc{0.0, 0.0};
-    for (int s = 0; s < A.nsplit; ++s) acc += A.part[(size_t)s * A.N + i];
-    A.ap[i] = acc * A.wd[i];
+    A.ap[i] = sum_parts(A, i) * A.wd[i];
 }
 
 // k_cg_jhv for NL candidates: one warp per CglCols columns, a CTA of 8
@@ -1113,6 +1243,7 @@ __global__ void __launch_bounds__(CGL_JH_NT, 2) k_cgl_jhv(CGLArgs L)
     static_assert(NL * NC <= 32, "one lane per (candidate, column)");
     using RT = typename JRaw<JP, JM>::T;
     __shared__ cd s_ap[2][NL][RC];
+    chain_wait();
     if (cgl_all_done(L)) return;   // the same for every thread of the grid
     const CGArgs& A = L.a;
     const size_t N = (size_t)A.N;
@@ -1214,6 +1345,34 @@ __global__ void __launch_bounds__(CGL_JH_NT, 2) k_cgl_jhv(CGLArgs L)
 
 }  // namespace
 
+// a launch with programmatic stream serialisation (chain_wait)
+template <typename... P, typename... V>
+static void chain(void (*kern)(P...), dim3 grid, int block, cudaStream_t s, V... v)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, P(v)...);
+}
+
+#define CRT_CG_CHAIN(KERNEL, GRID, BLOCK, STREAM)                                  \
+    do {                                                                           \
+        switch (a.jprec * 3 + a.jmode) {                                           \
+        case 0: chain(KERNEL<0, 0>, GRID, BLOCK, STREAM, a); break;                \
+        case 1: chain(KERNEL<0, 1>, GRID, BLOCK, STREAM, a); break;                \
+        case 2: chain(KERNEL<0, 2>, GRID, BLOCK, STREAM, a); break;                \
+        case 3: chain(KERNEL<1, 0>, GRID, BLOCK, STREAM, a); break;                \
+        case 4: chain(KERNEL<1, 1>, GRID, BLOCK, STREAM, a); break;                \
+        default: chain(KERNEL<1, 2>, GRID, BLOCK, STREAM, a); break;               \
+        }                                                                          \
+    } while (0)
+
 #define CRT_CG_DISPATCH(KERNEL, GRID, BLOCK, STREAM, ...)                          \
     do {                                                                           \
         const int key = a.jprec * 3 + a.jmode;                                     \
@@ -1233,7 +1392,17 @@ void launch_cg_setup(const CGArgs& a, const cd* dat, const cd* sigmaa, const cd*
     CRT_CG_DISPATCH(k_cg_setup, (a.M + cols_per_block - 1) / cols_per_block, SU_NT, s, a, dat, sigmaa, par);
 }
 
-void launch_cg_init(const CGArgs& a, cudaStream_t s) { k_cg_init<<<1, VEC_NT, 0, s>>>(a); }
+static void chain_head(const CGArgs& a, cudaStream_t s)
+{
+    chain(k_cg_head_sums, VS_CTAS, 32, s, a);
+    chain(k_cg_head_update, (a.M + VS_UPD_NT - 1) / VS_UPD_NT, VS_UPD_NT, s, a);
+}
+
+void launch_cg_init(const CGArgs& a, cudaStream_t s)
+{
+    k_cg_init<<<1, VEC_NT, 0, s>>>(a);
+    if (a.turn) chain_head(a, s);
+}
 
 namespace {
 // J^H pass with NC cells per warp (4; CRT_B200_JH_COLS=2 / 8 for the others)
@@ -1243,12 +1412,12 @@ void launch_cg_jhv_nc(const CGArgs& a, cudaStream_t s)
     const int cols_per_block = (JH_NT / 32) * NC;
     const int grid = (a.M + cols_per_block - 1) / cols_per_block;
     switch (a.jprec * 3 + a.jmode) {
-    case 0: k_cg_jhv<0, 0, NC><<<grid, JH_NT, 0, s>>>(a); break;
-    case 1: k_cg_jhv<0, 1, NC><<<grid, JH_NT, 0, s>>>(a); break;
-    case 2: k_cg_jhv<0, 2, NC><<<grid, JH_NT, 0, s>>>(a); break;
-    case 3: k_cg_jhv<1, 0, NC><<<grid, JH_NT, 0, s>>>(a); break;
-    case 4: k_cg_jhv<1, 1, NC><<<grid, JH_NT, 0, s>>>(a); break;
-    default: k_cg_jhv<1, 2, NC><<<grid, JH_NT, 0, s>>>(a); break;
+    case 0: chain(k_cg_jhv<0, 0, NC>, grid, JH_NT, s, a); break;
+    case 1: chain(k_cg_jhv<0, 1, NC>, grid, JH_NT, s, a); break;
+    case 2: chain(k_cg_jhv<0, 2, NC>, grid, JH_NT, s, a); break;
+    case 3: chain(k_cg_jhv<1, 0, NC>, grid, JH_NT, s, a); break;
+    case 4: chain(k_cg_jhv<1, 1, NC>, grid, JH_NT, s, a); break;
+    default: chain(k_cg_jhv<1, 2, NC>, grid, JH_NT, s, a); break;
     }
 }
 void launch_cg_jhv(const CGArgs& a, cudaStream_t s)
@@ -1288,7 +1457,7 @@ void launch_cg_fused(const CGArgs& a, cudaStream_t s)
 
 void launch_cg_iterations(const CGArgs& a, int iters, const SpcPlan* spc, Gnn* gnn, cd* zb, cudaStream_t s)
 {
-    const int nt = 256;
+    const int nt = 128;
     dim3 gjv((a.N + JV_NT - 1) / JV_NT, a.nsplit);
     const int gvec = (a.M + VS_UPD_NT - 1) / VS_UPD_NT;
     for (int it = 0; it < iters; ++it) {
@@ -1301,21 +1470,24 @@ void launch_cg_iterations(const CGArgs& a, int iters, const SpcPlan* spc, Gnn* g
             } else {
                 launch_gnn_apply(*gnn, a.r, nullptr, a.z, a.st, s);
             }
-            k_cg_head_pc_sums<<<VS_CTAS, 32, 0, s>>>(a);
-            k_cg_head_pc_update<<<gvec, VS_UPD_NT, 0, s>>>(a);
-        } else {
-            k_cg_head_sums<<<VS_CTAS, 32, 0, s>>>(a);
-            k_cg_head_update<<<gvec, VS_UPD_NT, 0, s>>>(a);
+            chain(k_cg_head_pc_sums, VS_CTAS, 32, s, a);
+            chain(k_cg_head_pc_update, gvec, VS_UPD_NT, s, a);
+        } else if (!a.turn) {
+            chain_head(a, s);
         }
         if (a.fused) {
             launch_cg_fused(a, s);
         } else {
-            CRT_CG_DISPATCH(k_cg_jv, gjv, JV_NT, s, a);
-            k_cg_jv_reduce<<<(a.N + nt - 1) / nt, nt, 0, s>>>(a);
+            CRT_CG_CHAIN(k_cg_jv, gjv, JV_NT, s);
+            chain(k_cg_jv_reduce, (a.N + nt - 1) / nt, nt, s, a);
             launch_cg_jhv(a, s);
         }
-        k_cg_tail_sums<<<VS_CTAS, 32, 0, s>>>(a);
-        k_cg_tail_update<<<gvec, VS_UPD_NT, 0, s>>>(a);
+        if (a.turn) {
+            chain(k_cg_turn, TURN_CTAS, TURN_NT, s, a);
+        } else {
+            chain(k_cg_tail_sums, VS_CTAS, 32, s, a);
+            chain(k_cg_tail_update, gvec, VS_UPD_NT, s, a);
+        }
     }
 }
 
@@ -1326,16 +1498,15 @@ void launch_cg_finish(const CGArgs& a, int lfpi, double step, cd* par, double* b
 
 // ---------------------------------------------------------------------------
 // Lambda candidates side by side.
-#define CRT_CGL_DISPATCH(KERNEL, NL, GRID, BLOCK, STREAM, ...)                     \
+#define CRT_CGL_DISPATCH(KERNEL, NL, GRID, BLOCK, STREAM)                          \
     do {                                                                           \
-        const int key = L.a.jprec * 3 + L.a.jmode;                                 \
-        switch (key) {                                                             \
-        case 0: KERNEL<0, 0, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break;  \
-        case 1: KERNEL<0, 1, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break;  \
-        case 2: KERNEL<0, 2, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break;  \
-        case 3: KERNEL<1, 0, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break;  \
-        case 4: KERNEL<1, 1, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break;  \
-        default: KERNEL<1, 2, NL><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
+        switch (L.a.jprec * 3 + L.a.jmode) {                                       \
+        case 0: chain(KERNEL<0, 0, NL>, GRID, BLOCK, STREAM, L); break;            \
+        case 1: chain(KERNEL<0, 1, NL>, GRID, BLOCK, STREAM, L); break;            \
+        case 2: chain(KERNEL<0, 2, NL>, GRID, BLOCK, STREAM, L); break;            \
+        case 3: chain(KERNEL<1, 0, NL>, GRID, BLOCK, STREAM, L); break;            \
+        case 4: chain(KERNEL<1, 1, NL>, GRID, BLOCK, STREAM, L); break;            \
+        default: chain(KERNEL<1, 2, NL>, GRID, BLOCK, STREAM, L); break;           \
         }                                                                          \
     } while (0)
 
@@ -1345,12 +1516,12 @@ template <int NL>
 void cgl_matvecs(const CGLArgs& L, cudaStream_t s)
 {
     const CGArgs& a = L.a;
-    const int nt = 256;
+    const int nt = 128;
     const dim3 gjv((a.N + JV_NT - 1) / JV_NT, a.nsplit);
-    CRT_CGL_DISPATCH(k_cgl_jv, NL, gjv, JV_NT, s, L);
-    k_cgl_jv_reduce<<<dim3((a.N + nt - 1) / nt, L.nl), nt, 0, s>>>(L);
+    CRT_CGL_DISPATCH(k_cgl_jv, NL, gjv, JV_NT, s);
+    chain(k_cgl_jv_reduce, dim3((a.N + nt - 1) / nt, L.nl), nt, s, L);
     const int cols_per_block = (CGL_JH_NT / 32) * CglCols<NL>::value;
-    CRT_CGL_DISPATCH(k_cgl_jhv, NL, (a.M + cols_per_block - 1) / cols_per_block, CGL_JH_NT, s, L);
+    CRT_CGL_DISPATCH(k_cgl_jhv, NL, (a.M + cols_per_block - 1) / cols_per_block, CGL_JH_NT, s);
 }
 
 }  // namespace
@@ -1362,21 +1533,24 @@ void launch_cgl_setup(const CGLArgs& L, const cd* dat, const cd* sigmaa, const c
     CRT_CG_DISPATCH(k_cgl_setup, (a.M + warps - 1) / warps, threads, s, L, dat, sigmaa, par);
 }
 
-void launch_cgl_init(const CGLArgs& L, cudaStream_t s) { k_cgl_init<<<L.nl, VEC_NT, 0, s>>>(L); }
+void launch_cgl_init(const CGLArgs& L, cudaStream_t s)
+{
+    k_cgl_init<<<L.nl, VEC_NT, 0, s>>>(L);
+    if (!L.a.pc) k_cgl_begin<<<L.nl, VEC_NT, 0, s>>>(L);   // the later heads come with the turns
+}
 
 int launch_cgl_iterations(const CGLArgs& L, int iters, cudaStream_t s)
 {
     for (int it = 0; it < iters; ++it) {
-        k_cgl_begin<<<L.nl, VEC_NT, 0, s>>>(L);
         if (L.nl <= 2)
             cgl_matvecs<2>(L, s);
         else if (L.nl <= 4)
             cgl_matvecs<4>(L, s);
         else
             cgl_matvecs<8>(L, s);
-        k_cgl_end<<<L.nl, VEC_NT, 0, s>>>(L);
+        chain(k_cgl_turn, TURN_CTAS * L.nl, TURN_NT, s, L);
     }
-    return 5 * iters;
+    return 4 * iters;
 }
 
 int launch_cgl_iteration_pc(const CGLArgs& L, cudaStream_t s)

@@ -56,6 +56,10 @@ struct CGArgs {
     unsigned long long* fepoch;   // [1] advanced by every iteration tail (tickets stay unique)
     int* ferr;                    // [1] set when a wait gave up
     int flag_lag;                 // row blocks between a block's two uses (CGF_S .. CGF_Q - 1)
+    // Jacobi form: one kernel ends an iteration and begins the next
+    // (k_cg_turn; the first head runs with launch_cg_init), instead of a tail
+    // and a head of two kernels each
+    int turn;
     double* vred;                 // [32][8] per-CTA partial sums of the grid-wide head and tail
 };
 
