@@ -53,26 +53,14 @@ template <> __device__ __forceinline__ cd shfl_t<cd>(cd v, int src)
     return cd{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
 }
 
-// Products by a reciprocal pivot and the pivot's root with every fused
-// multiply-add spelled out, so that the factor's bits do not hang on what the
-// compiler contracts here: the forms k_band_factor_blk compiles to, within its
-// diagonal block (`row` false) and in its rows below it.
+// Products by a reciprocal pivot in the forms k_band_factor_blk compiles to,
+// within its diagonal block (`row` false) and in its rows below it.
 __device__ __forceinline__ cd mul_inv(cd a, cd inv, bool row)
 {
     const double p = __dmul_rn(a.x, inv.y), q = __dmul_rn(a.y, inv.x);
     return cd{fma(a.x, inv.x, -__dmul_rn(a.y, inv.y)), row ? fma(a.y, inv.x, p) : fma(a.x, inv.y, q)};
 }
 __device__ __forceinline__ double mul_inv(double a, double inv, bool) { return a * inv; }
-// Sc<cd>::sqrt_recip
-__device__ __forceinline__ void pivot_root(cd z, cd& root, cd& inv)
-{
-    const double r2 = fma(z.x, z.x, __dmul_rn(z.y, z.y));
-    const double ir = rsqrt(r2), u = __dmul_rn(0.5, fma(r2, ir, fabs(z.x)));
-    const double iu = rsqrt(u), t = __dmul_rn(u, iu), h = __dmul_rn(0.5, iu);
-    root = z.x >= 0.0 ? cd{t, __dmul_rn(z.y, h)} : cd{__dmul_rn(fabs(z.y), h), copysign(t, z.y)};
-    inv = cd{__dmul_rn(root.x, ir), -__dmul_rn(root.y, ir)};
-}
-__device__ __forceinline__ void pivot_root(double z, double& root, double& inv) { Sc<double>::sqrt_recip(z, root, inv); }
 
 // fms_acc(acc, a, b), or fms_acc(acc, b, a) when rev: the imaginary part's two
 // products in the other order
@@ -184,7 +172,7 @@ __global__ void __launch_bounds__(32 * (NU + 1), 1) k_band_factor_mma(BandArgs<T
             if (t >= npp) break;
             if (Sc<T>::bad_pivot(piv)) s_err = CRT_ERR_PIVOT;
             T root, inv;
-            pivot_root(piv, root, inv);
+            root_fx(piv, root, inv);
             const T l = j == t ? root : mul_inv(t < 4 ? a0 : a1, inv, H4 && (j >> 2) != (t >> 2));
             if (t + 1 < FP) {
                 const T lr_ = shfl_t(l, (lane & ~3) | (t & 3));              // L(j, t)

@@ -156,6 +156,35 @@ CRT_HD void fms_acc(cf& acc, cf a, cf b)
 }
 CRT_HD cf scale(cf a, double s) { return cf{(float)(a.x * s), (float)(a.y * s)}; }
 
+// Product, pivot's root and reciprocal with every fused multiply-add spelled
+// out: which of two products the compiler contracts depends on the kernel
+// around them, and kernels that replace one another must give the same bits.
+__device__ __forceinline__ cd mul_fx(cd a, cd b)
+{
+    return cd{fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x))};
+}
+__device__ __forceinline__ double mul_fx(double a, double b) { return a * b; }
+// principal root and its reciprocal from two reciprocal square roots (Sc<cd>::sqrt_recip)
+__device__ __forceinline__ void root_fx(cd z, cd& root, cd& inv)
+{
+    const double r2 = fma(z.x, z.x, __dmul_rn(z.y, z.y));
+    const double ir = rsqrt(r2), u = __dmul_rn(0.5, fma(r2, ir, fabs(z.x)));
+    const double iu = rsqrt(u), t = __dmul_rn(u, iu), h = __dmul_rn(0.5, iu);
+    root = z.x >= 0.0 ? cd{t, __dmul_rn(z.y, h)} : cd{__dmul_rn(fabs(z.y), h), copysign(t, z.y)};
+    inv = cd{__dmul_rn(root.x, ir), -__dmul_rn(root.y, ir)};
+}
+__device__ __forceinline__ void root_fx(double z, double& root, double& inv)
+{
+    inv = rsqrt(z);
+    root = z * inv;
+}
+__device__ __forceinline__ cd recip_fx(cd a)
+{
+    const double s = 1.0 / fma(a.x, a.x, __dmul_rn(a.y, a.y));
+    return cd{__dmul_rn(a.x, s), -__dmul_rn(a.y, s)};
+}
+__device__ __forceinline__ double recip_fx(double a) { return 1.0 / a; }
+
 CRT_HD double scale(double a, double s) { return a * s; }
 CRT_HD cd scale(cd a, double s) { return cd{a.x * s, a.y * s}; }
 

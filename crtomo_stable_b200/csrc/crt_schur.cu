@@ -16,10 +16,10 @@
 //       in 4 x 4 register tiles;
 //   k_schur_gram    C = V^T [u^ | V^] per wavenumber (tiled GEMM on the FP64
 //       tensor pipe that skips the rows where a column is still zero);
-//   k_schur_chol    per (k, l): S_l = A_GG(l) - V^T V^, right-looking
-//       blocked Cholesky (unconjugated, complex symmetric as
-//       src/chol.f90:44-78) with a 16-column panel in shared memory, the
-//       forward solve fused into the factorisation, the back solve by panels;
+//   k_schur_ll      per (k, l): S_l = A_GG(l) - V^T V^, left-looking blocked
+//       Cholesky (unconjugated, complex symmetric as src/chol.f90:44-78), the
+//       forward solve fused into the factorisation, the back solve by panels
+//       (k_schur_chol, right-looking, for the largest complex boundaries);
 //   k_schur_zrebuild  z^ = u^ - V^ p_G (tiled GEMM);
 //   k_schur_out_gam p_G into kpot at the boundary nodes.
 #include "crt_schur.h"
@@ -937,6 +937,246 @@ __global__ void __launch_bounds__(NT, PF ? 1 : 2) k_schur_chol(SchurArgs s, Band
     for (int g = tid; g < m; g += NT) xg[(size_t)sys * m + g] = y[g];
 }
 
+// ---------------------------------------------------------------------------
+// The same factorisation left-looking, on the FP64 tensor pipe, a CTA per
+// system: per block column of 8, every 8 x 8 tile below the diagonal is
+// summed over the finished columns in registers (a warp per row block, m8n8k4
+// products in ascending columns), the diagonal block is factored by one warp
+// and the rows below are solved by a thread each; nothing is written twice.
+// The right-looking form's three barriers and shared-memory passes per column
+// and its trailing update through L2 took 4,900 cycles a column (m = 101,
+// complex).  Measured, all systems: 400 of m = 101 complex 0.50 -> 0.33 ms, 576
+// of 181 complex 1.43 -> 1.02, 1,152 of 253 real 3.23 -> 1.88; the reference
+// factors of 128 groups of 492: 3.4 -> 3.0.  The factor lies in shared memory where two CTAs share an SM
+// (SM), packed by block columns, else column-major in the workspace, its
+// finished block columns staged one ahead by cp.async.  Entries take their
+// updates in the same order and form as there, and the back solve keeps its
+// panels of NBP columns and their partial sums: the same bits.
+constexpr int LL_NT = 256;
+// entries of the packed factor: block columns of 8 padded runs (a product's k
+// columns x four rows in different banks)
+__host__ __device__ inline size_t ll_packed(int m)
+{
+    const size_t nbk = (m + 7) / 8;
+    return 8 * (nbk * (8 * nbk + 4) - 4 * nbk * (nbk - 1));
+}
+template <typename T> size_t ll_smem(int m, bool sm)
+{
+    const size_t m8 = (m + 7) / 8 * 8;
+    return (m8 * (8 + RunPad<T>::v) + m8 + (sm ? ll_packed(m) : 2 * 8 * (m8 + 4))) * sizeof(T);
+}
+
+template <typename T, bool SM, bool REF, int NT, int U>
+__global__ void __launch_bounds__(NT, 512 / NT) k_schur_ll(SchurArgs s, BandArgs<T> A, const T* __restrict__ C, T* Sws,
+                                                           T* xg, int sys0, int NBP, int* nonconv)
+{
+    constexpr int ST = 8 + RunPad<T>::v, NW = NT / 32;
+    using Tile = MmaTile<T>;
+    constexpr int KC = Tile::KC;
+    extern __shared__ __align__(16) unsigned char ll_dyn[];
+    const int m = s.m, nbk = (m + 7) / 8, m8 = 8 * nbk;
+    T* pan = reinterpret_cast<T*>(ll_dyn);   // [m8][ST] the block column before its solve
+    T* y = pan + (size_t)m8 * ST;            // [m8]
+    T* pack = y + m8;                        // the packed factor, or the two stages [8][m8 + 4]
+    __shared__ T LD[8][8], LDi[8], zb[8];    // LD[t][j] = L(c0 + j, c0 + t)
+    __shared__ int s_err;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.x, sys = sys0 + b;
+    const int k = REF ? b / s.ngrp : sys / s.L, l = REF ? (b % s.ngrp) * s.grp : sys % s.L;
+    T* S = Sws + (size_t)b * m * m;
+    const T* Ck = C + (size_t)k * s.ncol * m;
+    // block column J: entry (r, 8 J + t) at blk(J)[t ld(J) + r] (r >= 8 J)
+    auto ld = [&](int J) { return SM ? m8 - 8 * J + 4 : m; };
+    auto blk = [&](int J) -> T* {
+        // packed: block columns 0 .. J-1 take the sum of 8 (m8 - 8 j + 4)
+        return SM ? pack + 8 * (J * (m8 + 4) - 4 * J * (J - 1)) - 8 * J : S + (size_t)8 * J * m;
+    };
+    auto at = [&](int r, int c) -> T& { return blk(c >> 3)[(c & 7) * ld(c >> 3) + r]; };
+    if (tid == 0) s_err = 0;
+    // eight columns of loads in flight per thread
+    for (int J = 0; J < nbk; ++J) {
+        T* cp = blk(J);
+        const int lj = ld(J), nc = min(8, m - 8 * J);
+        const T* src = REF ? C + ((size_t)k * m + 8 * J) * m : Ck + (size_t)(s.L + 8 * J) * m;
+        for (int r = 8 * J + tid; r < m; r += NT) {
+            T v[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (t < nc && r >= 8 * J + t) v[t] = src[(size_t)t * m + r];
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (t < nc && r >= 8 * J + t) cp[t * lj + r] = REF ? v[t] : -v[t];   // REF: C is S0
+        }
+    }
+    for (int g = tid; g < m8; g += NT) {
+        T v = Sc<T>::zero();
+        if (!REF && g < m) {
+            v = -Ck[(size_t)l * m + g];
+            if (g == s.posG_src[l]) v += Sc<T>::one();
+            if (s.lsink && g == s.posG_sink) v -= Sc<T>::one();
+        }
+        y[g] = v;
+    }
+    __syncthreads();
+    if constexpr (REF) {
+        const int nl = min(s.grp, s.L - l);
+        for (int g = tid; g < m; g += NT)
+            for (int q = s.bd_ptr[g]; q < s.bd_ptr[g + 1]; ++q) {
+                const int h = s.bd_col[q];
+                if (h <= g) at(g, h) += band_assemble_part<T>(A, s.bd_ent[q], k, l, nl, 1);
+            }
+    } else {
+        for (int q = tid; q < s.ngg; q += NT) at(s.gg_g[q], s.gg_h[q]) += band_assemble_entry<T>(A, s.gg_ent[q], k, l);
+    }
+    __syncthreads();
+    const int lr = lane >> 2, lc = 2 * (lane & 3);
+    for (int J = 0; J < nbk; ++J) {
+        const int c0 = 8 * J, npp = min(8, m - c0), lj = ld(J);
+        T* cb = blk(J);
+        // block column K's rows from c0 on into stage K % 2
+        const int sl = m8 - c0 + 4;
+        auto stage = [&](int K) {
+            if (SM || K >= J) return;
+            const T* src = S + (size_t)8 * K * m;
+            T* dst = pack + (K & 1) * 8 * (m8 + 4) - c0;
+            for (int t = warp; t < 8; t += NW)
+                for (int r = c0 + lane; r < m; r += 32) cp_async_elem<T>(dst + t * sl + r, src + (size_t)t * m + r);
+        };
+        // tiles (I, J) minus the finished columns, U row blocks of a warp at a time
+        for (int I0 = J; I0 < nbk; I0 += U * NW) {
+            Tile acc[U];
+            int row[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int r = 8 * (I0 + warp + u * NW) + lr;
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    acc[u].set(q, r < m && c0 + lc + q <= r ? cb[(lc + q) * lj + r] : Sc<T>::zero());
+                row[u] = min(r, m - 1);   // rows past the end repeat the last one
+            }
+            const int rj = min(c0 + lr, m - 1), nu = min(U, (nbk - I0 - warp + NW - 1) / NW);
+            stage(0);
+            cp_async_commit();
+            for (int K = 0; K < J; ++K) {
+                const T* kc = SM ? blk(K) : pack + (K & 1) * 8 * (m8 + 4) - c0;
+                const int kl = SM ? ld(K) : sl;
+                if (!SM) {
+                    cp_async_wait_group<0>();
+                    __syncthreads();   // stage K has landed, stage K - 1's readers are through
+                    stage(K + 1);
+                    cp_async_commit();
+                }
+                kc += Tile::kk() * kl;
+#pragma unroll
+                for (int t = 0; t < 8; t += KC) {
+                    const typename Tile::B bf = Tile::ldb(kc + t * kl + rj);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (u < nu) acc[u].mma(Tile::lda_neg(kc + t * kl + row[u]), bf);
+                }
+            }
+            if (!SM) __syncthreads();   // the stages may be filled again
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (u < nu)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) pan[(8 * (I0 + warp + u * NW) + lr) * ST + lc + q] = acc[u].get(q);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // the diagonal block: lane 4 j + g holds row j's entries of columns
+            // g and g + 4, and y of its row
+            const int j = lane >> 2, g = lane & 3;
+            T a0 = pan[(c0 + j) * ST + g], a1 = pan[(c0 + j) * ST + g + 4], yj = y[c0 + j];
+            T piv = shfl_w(a0, 0, 32);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                if (t >= npp) break;
+                if (Sc<T>::bad_pivot(piv)) s_err = CRT_ERR_PIVOT;
+                T root, inv;
+                root_fx(piv, root, inv);
+                const T lt = j == t ? root : mul_fx(t < 4 ? a0 : a1, inv);
+                const T yc = mul_fx(yj, inv);
+                const T z = shfl_w(yc, 4 * t, 32);
+                const T lrow = shfl_w(lt, (lane & ~3) | (t & 3), 32);   // L(j, t)
+                if (j > t) fms_acc(yj, lrow, z);
+                if (t + 1 < 8) {
+                    if (t < 3) fms_acc(a0, lrow, shfl_w(lt, 4 * g + (t & 3), 32));
+                    fms_acc(a1, lrow, shfl_w(lt, 4 * (g + 4) + (t & 3), 32));
+                    piv = shfl_w(t + 1 < 4 ? a0 : a1, 4 * (t + 1) + ((t + 1) & 3), 32);
+                }
+                if (g == (t & 3) && j >= t && j < npp) {
+                    LD[t][j] = lt;
+                    cb[t * lj + c0 + j] = lt;
+                }
+                if (lane == 0) {
+                    LDi[t] = inv;
+                    zb[t] = z;
+                    y[c0 + t] = z;
+                }
+            }
+        }
+        __syncthreads();
+        if (s_err) break;
+        // the rows below (a full block: there are rows only then)
+        for (int r = c0 + 8 + tid; r < m; r += NT) {
+            const T* px = pan + r * ST;
+            T v[8], yr = REF ? Sc<T>::zero() : y[r];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v[t] = px[t];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                v[t] = mul_fx(v[t], LDi[t]);
+#pragma unroll
+                for (int t2 = t + 1; t2 < 8; ++t2) fms_acc(v[t2], v[t], LD[t][t2]);
+                if (!REF) fms_acc(yr, v[t], zb[t]);
+                cb[t * lj + r] = v[t];
+            }
+            if (!REF) y[r] = yr;
+        }
+        __syncthreads();
+    }
+    if constexpr (REF) {
+        if (s_err && tid == 0) atomicAdd(nonconv, 1);
+        return;
+    }
+    if (s_err) {
+        if (tid == 0) atomicMax(&s.status[sys], s_err);
+        return;
+    }
+    // L^T x = y, panel by panel from the last
+    for (int p0 = (m - 1) / NBP * NBP; p0 >= 0; p0 -= NBP) {
+        const int nb = min(NBP, m - p0);
+        {   // y[p0 + t] -= sum over solved rows r >= p0 + nb of L(r, p0 + t) x_r
+            const int t = tid >> 4, sl = tid & 15;   // NT = 256 here
+            T part = Sc<T>::zero();
+            if (t < nb) {
+                const T* cp = &at(0, p0 + t);
+#pragma unroll 4
+                for (int r = p0 + nb + sl; r < m; r += 16) fma_acc(part, cp[r], y[r]);
+            }
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) part += shfl_xor_t(part, off);
+            if (sl == 0 && t < nb) y[p0 + t] -= part;
+        }
+        __syncthreads();
+        if (warp == 0) {   // the panel's triangle of L^T, lane t = row p0 + t
+            const T* cl = &at(0, p0 + min(lane, nb - 1));
+            T v = lane < nb ? y[p0 + lane] : Sc<T>::zero();
+            const T rc = recip_fx(cl[p0 + min(lane, nb - 1)]);
+            for (int u = nb - 1; u >= 0; --u) {
+                const T lu = lane < u ? cl[p0 + u] : Sc<T>::zero();
+                if (lane == u) v = mul_fx(v, rc);
+                const T x = shfl_w(v, u, 32);
+                if (lane < u) fms_acc(v, lu, x);
+            }
+            if (lane < nb) y[p0 + lane] = v;
+        }
+        __syncthreads();
+    }
+    for (int g = tid; g < m; g += NT) xg[(size_t)sys * m + g] = y[g];
+}
+
 // |Re| + |Im| (the convergence test's magnitude)
 __device__ __forceinline__ double mag1(double a) { return fabs(a); }
 __device__ __forceinline__ double mag1(cd a) { return fabs(a.x) + fabs(a.y); }
@@ -1431,20 +1671,36 @@ void launch_schur_gram(const SchurArgs& s, const T* X, T* C, cudaStream_t st)
         go(k_schur_gram<T, 32, 16, 2, 1, 4>, 32, 16, 128, 4);
 }
 
+// columns per panel of the back solve (its partial sums' order): 12, or 16
+// above 553 complex boundary nodes
+template <typename T>
+static int ll_back_panel(int m) { return 2 * ((size_t)13 * m * sizeof(T) + 1024) <= 227 * 1024 ? 12 : 16; }
+
 template <typename T>
 void launch_schur_chol(const SchurArgs& s, const BandArgs<T>& full, const T* C, T* Sws, T* xg, int sys0, int nsys,
                        cudaStream_t st)
 {
-    // one CTA per SM with 16-column panels and the register prefetch, or two
-    // CTAs per SM with 12-column panels where two such panels fit
-    // (CRT_B200_SCHUR_CHOL=1 / 2 forces the form)
+    constexpr size_t lim = 227 * 1024;
+    auto go = [&](auto kern, size_t smem) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<nsys, LL_NT, smem, st>>>(s, full, C, Sws, xg, sys0, ll_back_panel<T>(s.m), nullptr);
+    };
+    // the factor in shared memory where two CTAs fit an SM (complex m = 101,
+    // 400 systems: 0.33 against 0.34 ms staged; real m = 181 with one CTA per
+    // SM 0.50 against 0.54)
+    if (2 * (ll_smem<T>(s.m, true) + 2048) <= lim) {
+        go(k_schur_ll<T, true, false, LL_NT, 4>, ll_smem<T>(s.m, true));
+        return;
+    }
+    if (ll_smem<T>(s.m, false) <= lim) {
+        go(k_schur_ll<T, false, false, LL_NT, 4>, ll_smem<T>(s.m, false));
+        return;
+    }
+    // above 536 complex boundary nodes the stages do not fit: right-looking,
+    // two CTAs per SM with 12-column panels up to 553, else one with 16
     constexpr int NT = 256;
     const size_t smem16 = ((size_t)16 * s.m + s.m) * sizeof(T), smem12 = ((size_t)12 * s.m + s.m) * sizeof(T);
-    const char* ev = std::getenv("CRT_B200_SCHUR_CHOL");
-    bool two = 2 * (smem12 + 1024) <= 227 * 1024;
-    if (ev && std::strcmp(ev, "1") == 0) two = false;
-    if (ev && std::strcmp(ev, "2") == 0 && 2 * (smem12 + 1024) <= 227 * 1024) two = true;
-    if (two) {
+    if (ll_back_panel<T>(s.m) == 12) {
         auto kern = k_schur_chol<T, NT, 12, false>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem12);
         kern<<<nsys, NT, smem12, st>>>(s, full, C, Sws, xg, sys0, nullptr);
@@ -1467,10 +1723,17 @@ void launch_schur_s0(const SchurArgs& s, const BandArgs<T>& full, const T* C, T*
 template <typename T>
 void launch_schur_ref(const SchurArgs& s, const BandArgs<T>& full, const T* S0, T* Lref, int* nonconv, cudaStream_t st)
 {
+    const int nref = s.K * s.ngrp;
+    const size_t smem = ll_smem<T>(s.m, false);
+    if (smem <= 227 * 1024) {
+        auto kern = k_schur_ll<T, false, true, 512, 4>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<nref, 512, smem, st>>>(s, full, S0, Lref, nullptr, 0, 0, nonconv);
+        return;
+    }
     constexpr int NT = 256;
     const size_t smem12 = ((size_t)12 * s.m + s.m) * sizeof(T), smem16 = ((size_t)16 * s.m + s.m) * sizeof(T);
-    const int nref = s.K * s.ngrp;
-    if (2 * (smem12 + 1024) <= 227 * 1024) {
+    if (ll_back_panel<T>(s.m) == 12) {
         auto kern = k_schur_chol<T, NT, 12, false, true>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem12);
         kern<<<nref, NT, smem12, st>>>(s, full, S0, Lref, nullptr, 0, nonconv);

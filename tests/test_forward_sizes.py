@@ -63,3 +63,24 @@ def test_factor_in_registers_is_the_panel_blocked_factor(nx, nz, panel, monkeypa
         ctx.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solve", ["direct", "iter"])
+@pytest.mark.parametrize("ldc", [False, True])
+@pytest.mark.parametrize("nx,nz,nel", [(5, 2, 2), (12, 5, 9), (30, 12, 17), (80, 40, 6), (150, 90, 5), (380, 80, 3)])
+def test_boundary_systems(nx, nz, nel, ldc, solve, monkeypatch):
+    """The electrodes' boundary systems (9 to 541 nodes: the factor in shared
+    memory, staged, and above the staged form's 536 complex nodes) by their
+    Cholesky factors and by the preconditioned iteration, against the oracle."""
+    from crtomo_stable_b200.lib import FORWARD_SCHUR, Context
+    from oracle.oracle import OracleProblem
+    mesh, enr, strnr, vnr, sigma = survey(nx, nz, nel, False)
+    kwn, kwnwi = np.array([0.02, 0.3]), np.array([0.1, 0.2])
+    monkeypatch.setenv("CRT_B200_SCHUR_SOLVE", solve)
+    ctx = Context(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=kwnwi)
+    kp = ctx.forward(sigma, ldc=ldc, want_kpot=True)[2]
+    assert ctx.forward_info()[0] == FORWARD_SCHUR
+    kp_o = OracleProblem(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=kwnwi).forward(sigma, ldc=ldc, nthreads=8)
+    assert np.abs(kp - kp_o).max() <= RTOL * np.abs(kp_o).max()
+    ctx.close()
