@@ -639,20 +639,8 @@ extern "C" crt_ctx* crt_create(int32_t device, const crt_mesh* mesh, const crt_s
         for (int rel : mixed_rel)
             for (int q = 0; q < 2; ++q) gnodes.push_back(nrel0[(size_t)(m.elanz + rel) * m.maxnodes + q]);
         SchurHost& H = ctx->schur_h;
-        // forward-sweep column blocks: 16 columns (two CTAs per SM with the
-        // rows one block ahead: 11.0 ms after the factor on the 60k-triangle
-        // mesh) or 32 (one CTA per SM, 11.7 ms; CRT_B200_SCHUR_R=32)
-        // (16 also where the 32-column block's buffers exceed shared memory)
-        const char* rv = std::getenv("CRT_B200_SCHUR_R");
-        int sweep_r = (rv && std::strcmp(rv, "32") == 0) ? SCHUR_MS_R : 16;
-        int plan_e = schur_plan_host(lists, ctx->n, gnodes, enr0, ctx->lsink, ctx->nsink - 1, H, sweep_r);
-        if (plan_e == CRT_OK && sweep_r != 16 && schur_sweep_smem<cd>(H.mbI, H.mbI + 1, sweep_r) > 227 * 1024) {
-            sweep_r = 16;
-            H = SchurHost{};
-            plan_e = schur_plan_host(lists, ctx->n, gnodes, enr0, ctx->lsink, ctx->nsink - 1, H, sweep_r);
-        }
-        if (plan_e == CRT_OK &&
-            schur_sweep_smem<cd>(H.mbI, H.mbI + 1, sweep_r) <= 227 * 1024 &&
+        const int plan_e = schur_plan_host(lists, ctx->n, gnodes, enr0, ctx->lsink, ctx->nsink - 1, H);
+        if (plan_e == CRT_OK && schur_sweep_smem<cd>(H.mbI, H.mbI + 1) <= 227 * 1024 &&
             (size_t)(16 + 1) * H.m * sizeof(cd) <= 227 * 1024 && band_factor_smem<cd>(H.mbI + 1) <= 227 * 1024) {
             auto up = [&](int** d, const std::vector<int>& v) {
                 const std::vector<int> one(1, 0);
@@ -685,7 +673,6 @@ extern "C" crt_ctx* crt_create(int32_t device, const crt_mesh* mesh, const crt_s
             S.ncol = ctx->L + H.m;
             S.mbI = H.mbI;
             S.nblk = (int)H.blk_start.size();
-            S.R = H.R;
             S.ncpl = (int)H.gi_pos.size();
             S.ngg = (int)H.gg_ent.size();
             S.permI = p_permI;

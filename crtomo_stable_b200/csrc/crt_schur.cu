@@ -6,14 +6,10 @@
 //       solves, and the coupling values a(g, i) kept for later steps;
 //   k_schur_transpose  the interior factor reversed and row-packed, so the
 //       back substitution runs as a forward sweep;
-//   k_schur_sweep   banded triangular sweep of R columns per CTA (forward for
+//   k_schur_sweep   banded triangular sweep of 16 columns per CTA (forward for
 //       all columns, each block from its first non-zero row; back for the
-//       source columns): the factor streams through shared memory in blocks
-//       of 16 columns (one bulk copy each, double-buffered, bounded
-//       mbarrier wait), the right-hand sides in a window of rows that arrive
-//       by cp.async two blocks ahead; per block a 16-row triangle (half-warp
-//       per column, shuffle broadcasts) and an (mb x 16) x (16 x R) update
-//       in 4 x 4 register tiles;
+//       source columns), the triangle of a block beside the update by the
+//       block before on the FP64 tensor pipe;
 //   k_schur_gram    C = V^T [u^ | V^] per wavenumber (tiled GEMM on the FP64
 //       tensor pipe that skips the rows where a column is still zero);
 //   k_schur_ll      per (k, l): S_l = A_GG(l) - V^T V^, left-looking blocked
@@ -30,15 +26,15 @@
 #include <algorithm>
 #include <cstdio>
 #include <numeric>
+#include <type_traits>
 #include <utility>
 
 // ---------------------------------------------------------------------------
 // Host plan.
 int schur_plan_host(const AssemblyLists& full, int n, const std::vector<int>& gamma_nodes,
-                    const std::vector<int>& enr0, int lsink, int nsink0, SchurHost& o, int R)
+                    const std::vector<int>& enr0, int lsink, int nsink0, SchurHost& o)
 {
     o = SchurHost{};
-    o.R = R;
     o.n = n;
     o.L = (int)enr0.size();
     std::vector<int> posI(n, -1), posG(n, -1);
@@ -146,7 +142,7 @@ int schur_plan_host(const AssemblyLists& full, int n, const std::vector<int>& ga
     o.col_order.resize(ncol);
     std::iota(o.col_order.begin(), o.col_order.end(), 0);
     std::stable_sort(o.col_order.begin(), o.col_order.end(), [&](int a, int b) { return first[a] < first[b]; });
-    for (int b0 = 0; b0 < ncol; b0 += R) {
+    for (int b0 = 0; b0 < ncol; b0 += SCHUR_MS_R) {
         const int f = first[o.col_order[b0]];
         o.blk_start.push_back(f >= o.nI ? o.nI : f / SCHUR_MS_BB * SCHUR_MS_BB);
     }
@@ -237,35 +233,77 @@ __global__ void k_schur_transpose(SchurArgs s, const T* __restrict__ Lws, T* Lre
 }
 
 // ---------------------------------------------------------------------------
-// Banded lower-triangular sweep L z = b for R columns per CTA: grid (column
-// blocks, K).  The factor's columns stream through shared memory BB at a
-// time (one bulk copy each, double-buffered, bounded mbarrier wait); the
-// right-hand sides live in a window Z[WZ][R] (row r at slot r mod WZ,
-// WZ >= mb + 3 BB), their rows arriving by cp.async two blocks ahead of
-// use.  Per block: the BB x BB triangle (one half-warp per column, shuffle
-// broadcasts, lane t holding row t), the finished rows out, and the
-// (mb x BB) x (BB x R) update of the rows below (4 x TC register tiles).
+// Banded lower-triangular sweep L z = b for SW_R columns per CTA: grid (K,
+// column blocks).  The factor's columns stream through shared memory SW_BB at
+// a time (one bulk copy each, NB buffers, bounded mbarrier wait), the
+// right-hand sides live in a window Z of WZ rows (row r at slot r mod WZ, WZ
+// >= mb + 3 SW_BB), their rows arriving by cp.async two blocks ahead of use.
+// Per block b (rows c0 .. c0 + 15), between barriers:
+//   A. warps 0 and 1 solve the block's triangle for eight columns each (a lane
+//      per column, 8 x 8 triangles in registers, the product between them on
+//      the tensor pipe) while the other warps take block b - 1's columns into
+//      the rows past block b;
+//   B. four warps take block b's columns into block b + 1's rows, a tile each,
+//      another starts the next factor copy, the rest write block b's rows out.
+// The updates are m8n8k4 FP64 tensor products.  Every row takes its columns
+// in ascending order by fused multiply-adds in fms_acc's order.  Bound by the
+// block's chain: 4,900 cycles at a half-bandwidth of 128 (phase A 3,800, its
+// products alone 2,050 on the FP64 pipe; B 700), 2,900 at 21.  As 4 x 2
+// multiply-add tiles per thread and a half-warp per triangle column it was
+// 11,800 (back sweep of 128 sources, 492 electrodes: 11.2 -> 4.7 ms; 101 at
+// a half-bandwidth of 21: 0.38 -> 0.13).
 //   back == 0: forward sweep of X's columns (col_order, from each block's
 //     first non-zero row), in place;
 //   back == 1: the back sweep L^T x^ = z^ of the source columns: Lws holds
 //     the reversed row-packed factor and the rows are read reversed; the
 //     solution goes out as kpot = fak x^ at the interior rows' nodes.
-template <typename T, int NT, int R, int BB, int TC = 4, int MINB = 1>
-__global__ void __launch_bounds__(NT, MINB) k_schur_sweep(SchurArgs s, const T* __restrict__ Lws,
-                                                          const double* __restrict__ fakws, T* X, cd* kpot, int n_kpot,
-                                                          int WZ, int back, int ahead = 2)
+constexpr int SW_R = SCHUR_MS_R, SW_BB = SCHUR_MS_BB;
+
+// Rows of the window are padded so that the eight rows of a tile differ in banks.
+template <typename T> struct SweepRow { static constexpr int v = SW_R + (sizeof(T) == 16 ? 1 : 4); };
+
+// Operands of the sweep's products: the factor's entry negated once for both
+// chains of a complex product, the sign between them with the solution's.
+template <typename T> struct SweepTile;
+template <> struct SweepTile<cd> : MmaTile<cd> {
+    __device__ __forceinline__ static double lda_neg(const cd* a)
+    {
+        return -reinterpret_cast<const double*>(a)[threadIdx.x & 1];
+    }
+    __device__ __forceinline__ static B ldb(const cd* b)
+    {
+        const double* p = reinterpret_cast<const double*>(b);
+        const double v = p[threadIdx.x & 1];
+        return B{(threadIdx.x & 1) ? -v : v, p[(threadIdx.x & 1) ^ 1]};
+    }
+    __device__ __forceinline__ void mma(double a, const B& b)
+    {
+        dmma(x0, x1, a, b.n);
+        dmma(y0, y1, a, b.s);
+    }
+};
+template <> struct SweepTile<double> : MmaTile<double> {};
+
+template <typename T, int NT, int NB, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+    k_schur_sweep(SchurArgs s, const T* __restrict__ Lws, const double* __restrict__ fakws, T* X, cd* kpot, int n_kpot,
+                  int WZ, int back)
 {
-    static_assert(BB == 16 && R % 4 == 0 && R <= 32 && NT % 32 == 0 && NT >= R && (TC == 4 || TC == 2),
-                  "sweep layout");
+    constexpr int R = SW_R, BB = SW_BB, RS = SweepRow<T>::v;
+    constexpr int NU = NT / 32 - 2;                              // update warps
+    constexpr int FW = 4, OT = NT - 32 * (FW + 1), NE = (BB * R + OT - 1) / OT;   // phase B: the fetching warp; threads and entries of the rows out
+    static_assert(NU >= 4 && OT >= 32, "warps of phase B: four tiles, one to fetch, the others the rows out");
+    using Tile = SweepTile<T>;
+    constexpr int KC = Tile::KC;
     extern __shared__ __align__(16) unsigned char sw_dyn[];
     const int W = s.WI, n = s.nI, mb = s.mbI;
-    T* Lb = reinterpret_cast<T*>(sw_dyn);   // [2][BB * W]
-    T* Z = Lb + 2 * BB * W;                 // [WZ][R]
-    __shared__ T dinv[BB];
+    T* Lb = reinterpret_cast<T*>(sw_dyn);   // [NB][BB * W]
+    T* Z = Lb + NB * BB * W;                // [WZ][RS]
+    __shared__ T dinv[2][BB];
     __shared__ int colid[R];
-    __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ __align__(8) unsigned long long bar[NB];
     __shared__ int s_err;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // wavenumbers along x: the CTAs start in the order of their blocks'
     // first rows, longest passes first over all wavenumbers
     const int blk = blockIdx.y, k = s.k0 + blockIdx.x;
@@ -278,372 +316,232 @@ __global__ void __launch_bounds__(NT, MINB) k_schur_sweep(SchurArgs s, const T* 
     }
     if (tid == 0) {
         s_err = 0;
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int q = 0; q < NB; ++q) mbar_init(&bar[q], 1);
     }
     __syncthreads();
-    int ph0 = 0, ph1 = 0;
-    auto colp = [&](int j) { return X + ((size_t)k * s.ncol + colid[j]) * n; };
-    auto fetch = [&](int c0, int buf) {
-        if (tid == 0) {
-            if (s.progress && !s_err) {
-                // the factor's columns [c0, c0 + BB) are final once its
-                // progress passes them.  The wait gives up after about 4 s,
-                // or at once when another CTA of this wavenumber gave up
-                // (status set); the result is then flagged as failed.
-                const int want = min(n, c0 + BB);
-                long polls = 0;
-                int got;
-                while (true) {
-                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(got) : "l"(s.progress + k) : "memory");
-                    if (got >= want) break;
-                    if (*(volatile const int*)(s.status + k) != 0 || ++polls > (1L << 22)) {
-                        s_err = 1;
-                        atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
-                        break;
-                    }
-                    __nanosleep(256);
+    auto fetch = [&](int c0, int buf) {   // by one thread
+        if (s.progress && !s_err) {
+            // the factor's columns [c0, c0 + BB) are final once its
+            // progress passes them.  The wait gives up after about 4 s,
+            // or at once when another CTA of this wavenumber gave up
+            // (status set); the result is then flagged as failed.
+            const int want = min(n, c0 + BB);
+            long polls = 0;
+            int got;
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(got) : "l"(s.progress + k) : "memory");
+                if (got >= want) break;
+                if (*(volatile const int*)(s.status + k) != 0 || ++polls > (1L << 22)) {
+                    s_err = 1;
+                    atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
+                    break;
                 }
-                // the copy below reads them through the async proxy
-                asm volatile("fence.proxy.async.global;\n" ::: "memory");
+                __nanosleep(256);
             }
-            const int bytes = min(BB, n - c0) * W * (int)sizeof(T);
-            mbar_expect_tx(&bar[buf], bytes);
-            bulk_g2s(Lb + (size_t)buf * BB * W, Lk + (size_t)c0 * W, bytes, &bar[buf]);
+            // the copy below reads them through the async proxy
+            asm volatile("fence.proxy.async.global;\n" ::: "memory");
         }
+        const int bytes = min(BB, n - c0) * W * (int)sizeof(T);
+        mbar_expect_tx(&bar[buf], bytes);
+        bulk_g2s(Lb + (size_t)buf * BB * W, Lk + (size_t)c0 * W, bytes, &bar[buf]);
     };
-    auto wait = [&](int buf) {
-        int& ph = buf ? ph1 : ph0;
-        if (!mbar_wait(&bar[buf], ph)) s_err = 1;
-        ph ^= 1;
-    };
-    // rows [r0, r1) of every column into their slots, one commit group
-    auto issue_rows = [&](int r0, int r1) {
-        const int nr = r1 - r0;
-        for (int idx = tid; idx < nr * R; idx += NT) {
-            const int j = idx / nr, r = r0 + idx % nr;
-            T* dst = Z + (size_t)(r % WZ) * R + j;
-            if (colid[j] >= 0) cp_async_elem<T>(dst, colp(j) + (back ? n - 1 - r : r));
-            else *dst = Sc<T>::zero();
-        }
-        cp_async_commit();
-    };
-    // rows arrive `ahead` blocks before use: 2 (WZ >= mb + 3 BB, the wait at
-    // the end of a block leaves one group in flight) or 1 (WZ >= mb + 2 BB,
-    // the rows issued at the start of a block awaited at its end: the
-    // smaller window lets two CTAs share an SM)
-    issue_rows(start, min(n, start + BB + mb));
-    if (ahead == 2) issue_rows(min(n, start + BB + mb), min(n, start + 2 * BB + mb));
-    fetch(start, 0);
-    if (ahead == 2) cp_async_wait_group<1>();
-    else cp_async_wait_group<0>();
-    __syncthreads();
-    int buf = 0;
-    for (int c0 = start; c0 < n; c0 += BB) {
-        const int nb = min(BB, n - c0);
-        wait(buf);
-        if (c0 + BB < n) fetch(c0 + BB, buf ^ 1);
-        // the rows `ahead` blocks ahead (their slots held rows finished a block ago)
-        issue_rows(min(n, c0 + (ahead + 1) * BB + mb - BB), min(n, c0 + (ahead + 1) * BB + mb));
-        const T* Lc = Lb + (size_t)buf * BB * W;
-        if (tid < nb) dinv[tid] = Sc<T>::recip(Lc[tid * W]);
-        __syncthreads();
-        // the block's rows sit in consecutive slots (WZ is a multiple of BB)
-        const int sb = c0 % WZ;
-        {   // the block's triangle: a half-warp per column, lane t holds row t
-            // and its row of the block's L in registers; at step u lane u
-            // finishes its row and hands it to the half-warp by a shuffle, so
-            // every row takes z_t -= L_tu z_u for u = 0 .. t-1, then z_t *= 1/L_tt
-            constexpr int HW = NT / 16;   // half-warps of the CTA (NT is a multiple of 32)
-            const int hw = tid >> 4, lt = tid & 15;
-            for (int j0 = 0; j0 < R; j0 += HW) {
-                const int j = j0 + hw;
-                const bool act = j < R && lt < nb;
-                T zt = Sc<T>::zero(), lrow[BB];
-#pragma unroll
-                for (int u = 0; u < BB; ++u)
-                    lrow[u] = (act && u < lt && lt - u <= mb) ? Lc[u * W + (lt - u)] : Sc<T>::zero();
-                if (act) zt = Z[(size_t)(sb + lt) * R + j];
-#pragma unroll
-                for (int u = 0; u < BB; ++u) {
-                    if (u < nb) {
-                        if (lt == u) zt = Sc<T>::mul(zt, dinv[u]);
-                        const T zu = shfl_w<T>(zt, u, 16);
-                        if (lt > u && lt < nb && lt - u <= mb) fms_acc(zt, lrow[u], zu);
-                    }
-                }
-                if (act) Z[(size_t)(sb + lt) * R + j] = zt;
-            }
-        }
-        __syncthreads();
-        // the block's rows are final: out
-        for (int idx = tid; idx < nb * R; idx += NT) {
-            const int j = idx / nb, t = idx % nb;
-            if (colid[j] < 0) continue;
-            const int r = c0 + t;
-            const T v = Z[(size_t)(sb + t) * R + j];
-            if (!back) {
-                colp(j)[r] = v;
-            } else {
-                const int i = n - 1 - r;
-                kpot[((size_t)k * s.L + colid[j]) * n_kpot + s.permI[i]] =
-                    Sc<T>::to_cd(scale(v, fakws[(size_t)k * n + i]));
-            }
-        }
-        {   // rows [c0 + nb, c0 + nb + mb) take the block's columns: a thread
-            // owns rows rq + NQ a (4 of them) and columns jq + (R/TC) c (TC of
-            // them), so a warp's loads fall on consecutive words; every entry
-            // takes the block's columns u = 0 .. nb-1 in order, whatever TC
-            const int rlo = c0 + nb, rhi = min(n, c0 + nb + mb);
-            const int NQ = (rhi - rlo + 3) >> 2;
-            constexpr int RJ = R / TC;
-            for (int tile = tid; tile < NQ * RJ; tile += NT) {
-                const int rq = tile / RJ, jq = tile % RJ;
-                T acc[4][TC];
-                int sl[4];
-#pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    const int r = rlo + rq + NQ * a;
-                    sl[a] = r < rhi ? r % WZ : -1;
-#pragma unroll
-                    for (int c = 0; c < TC; ++c)
-                        acc[a][c] = sl[a] >= 0 ? Z[(size_t)sl[a] * R + jq + RJ * c] : Sc<T>::zero();
-                }
-#pragma unroll
-                for (int u = 0; u < BB; ++u) {
-                    if (u < nb) {
-                        T zc[TC], lv[4];
-#pragma unroll
-                        for (int c = 0; c < TC; ++c) zc[c] = Z[(size_t)(sb + u) * R + jq + RJ * c];
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            const int d = rlo + rq + NQ * a - (c0 + u);
-                            lv[a] = (sl[a] >= 0 && d <= mb) ? Lc[u * W + d] : Sc<T>::zero();
-                        }
-#pragma unroll
-                        for (int a = 0; a < 4; ++a)
-#pragma unroll
-                            for (int c = 0; c < TC; ++c) fms_acc(acc[a][c], lv[a], zc[c]);
-                    }
-                }
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-                    if (sl[a] >= 0)
-#pragma unroll
-                        for (int c = 0; c < TC; ++c) Z[(size_t)sl[a] * R + jq + RJ * c] = acc[a][c];
-            }
-        }
-        // the buffer just read is the destination of the bulk copy after next
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        if (ahead == 2) cp_async_wait_group<1>();   // the rows of the next block have landed
-        else cp_async_wait_group<0>();
-        __syncthreads();
-        buf ^= 1;
-    }
-    cp_async_wait_group<0>();
-    if (tid == 0 && s_err) atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
-}
-
-// ---------------------------------------------------------------------------
-// The sweeps with R = 16 columns per CTA (512 threads) and the triangle
-// beside the update (back: the source columns of the back sweep; forward:
-// the 16-column blocks of the forward sweep, CRT_B200_SCHUR_R=16): per block b (rows c0 .. c0 + 16), between
-// barriers,
-//   A. warps 0-7 solve block b's triangle (a half-warp per column, lane t
-//      holding row t; the finished row handed on by a shuffle) while warps
-//      8-15 take block b-1's columns into the rows past block b (those of
-//      block b took them in phase B of block b-1);
-//   B. threads 0-255 take block b's columns into block b+1's rows (an entry
-//      each) while warps 8-15 write block b's rows out.
-// Every row takes the blocks' columns in block order and each block's
-// columns in order, with the operations of k_schur_sweep; the factor's
-// column blocks b-1, b, b+1 sit in three buffers.
-template <typename T>
-__global__ void __launch_bounds__(512, 1) k_schur_sweep_pp(SchurArgs s, const T* __restrict__ Lws,
-                                                         const double* __restrict__ fakws, T* X, cd* kpot,
-                                                         int n_kpot, int WZ, int back)
-{
-    constexpr int R = 16, BB = 16, NT = 512, TC = 2;
-    extern __shared__ __align__(16) unsigned char bp_dyn[];
-    const int W = s.WI, n = s.nI, mb = s.mbI;
-    T* Lb = reinterpret_cast<T*>(bp_dyn);   // [3][BB * W]
-    T* Z = Lb + 3 * BB * W;                 // [WZ][R]
-    __shared__ T dinv[BB];
-    __shared__ int colid[R];
-    __shared__ __align__(8) unsigned long long bar[3];
-    __shared__ int s_err;
-    const int tid = threadIdx.x;
-    const int blk = blockIdx.y, k = s.k0 + blockIdx.x;
-    const int start = back ? 0 : s.blk_start[blk];
-    if (start >= n) return;   // every column of the block is zero, and so is its solution
-    const T* Lk = Lws + (size_t)k * n * W;
-    if (tid < R) {
-        const int c = blk * R + tid;
-        colid[tid] = back ? (c < s.L ? c : -1) : (c < s.ncol ? s.col_order[c] : -1);
-    }
-    if (tid == 0) {
-        s_err = 0;
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_init(&bar[2], 1);
-    }
-    __syncthreads();
-    int phs = 0;
-    auto fetch = [&](int c0, int buf) {
-        if (tid == 0) {
-            if (s.progress && !s_err) {
-                // beside the factor: its columns [c0, c0 + BB) are final once
-                // its progress passes them (bounded wait, as k_schur_sweep)
-                const int want = min(n, c0 + BB);
-                long polls = 0;
-                int got;
-                while (true) {
-                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(got) : "l"(s.progress + k) : "memory");
-                    if (got >= want) break;
-                    if (*(volatile const int*)(s.status + k) != 0 || ++polls > (1L << 22)) {
-                        s_err = 1;
-                        atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
-                        break;
-                    }
-                    __nanosleep(256);
-                }
-                asm volatile("fence.proxy.async.global;\n" ::: "memory");
-            }
-            const int bytes = min(BB, n - c0) * W * (int)sizeof(T);
-            mbar_expect_tx(&bar[buf], bytes);
-            bulk_g2s(Lb + (size_t)buf * BB * W, Lk + (size_t)c0 * W, bytes, &bar[buf]);
-        }
-    };
-    auto wait = [&](int buf) {
-        if (!mbar_wait(&bar[buf], (phs >> buf) & 1)) s_err = 1;
-        phs ^= 1 << buf;
+    // the reciprocals of a block's diagonal, by one warp once its copy has landed
+    auto pivots = [&](int buf, int phase, T* di) {
+        if (!mbar_wait(&bar[buf], phase)) s_err = 1;
+        if (lane < BB) di[lane] = recip_fx(Lb[(size_t)(buf * BB + lane) * W]);
     };
     auto colp = [&](int j) { return X + ((size_t)k * s.ncol + colid[j]) * n; };   // the column's rows in X
-    auto issue_rows = [&](int r0, int r1) {
-        const int nr = r1 - r0;
-        for (int idx = tid; idx < nr * R; idx += NT) {
-            const int j = idx / nr, r = r0 + idx % nr;
-            T* dst = Z + (size_t)(r % WZ) * R + j;
-            if (colid[j] >= 0) cp_async_elem<T>(dst, colp(j) + (back ? n - 1 - r : r));
-            else *dst = Sc<T>::zero();
-        }
-        cp_async_commit();
+    auto copy_row = [&](int j, int r, T* dst) {
+        if (colid[j] >= 0) cp_async_elem<T>(dst, colp(j) + (back ? n - 1 - r : r));
+        else *dst = Sc<T>::zero();
     };
-    // rows [rlo, rhi) take the columns of the block at cb (nbb rows, factor
-    // block Lq), threads [t0, t0 + nt): 4 rows x TC columns per thread
-    auto update_rows = [&](const T* Lq, int cb, int nbb, int rlo, int rhi, int t0, int nt) {
-        if (rlo >= rhi) return;
-        const int NQ = (rhi - rlo + 3) >> 2;
-        constexpr int RJ = R / TC;
-        const int sbb = cb % WZ;
-        for (int tile = tid - t0; tile < NQ * RJ; tile += nt) {
-            const int rq = tile / RJ, jq = tile % RJ;
-            T acc[4][TC];
-            int sl[4];
+    const int lr = lane >> 2, lg = lane & 3;
+    // NR tiles of 8 rows (slots sr and, `step` slots on, sr2) x NC tiles of 8
+    // columns from column j0 minus a factor block Lq whose solution rows begin
+    // at slot sb; the tiles' rows are d0, d0 + step below the block's first
+    // row, and those from dhi on are left as they are
+    auto update = [&](auto nr_, auto nc_, const T* Lq, int sb, const int* sr, int d0, int step, int dhi, int j0) {
+        constexpr int NR = decltype(nr_)::value, NC = decltype(nc_)::value;
+        Tile acc[NR][NC];
+        T* zp[NR];
+        const T* ap[NR];
+        const int kk = Tile::kk();
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const int r = rlo + rq + NQ * a;
-                sl[a] = r < rhi ? r % WZ : -1;
+        for (int a = 0; a < NR; ++a) {
+            zp[a] = Z + (size_t)(sr[a] + lr) * RS + j0 + 2 * lg;
+            ap[a] = Lq + kk * (W - 1) + d0 + a * step + lr;   // column u is u (W - 1) on
 #pragma unroll
-                for (int c = 0; c < TC; ++c)
-                    acc[a][c] = sl[a] >= 0 ? Z[(size_t)sl[a] * R + jq + RJ * c] : Sc<T>::zero();
-            }
+            for (int c = 0; c < NC; ++c)
 #pragma unroll
-            for (int u = 0; u < BB; ++u) {
-                if (u < nbb) {
-                    T zc[TC], lv[4];
+                for (int q = 0; q < 2; ++q) acc[a][c].set(q, zp[a][8 * c + q]);
+        }
+        const T* bp = Z + (size_t)(sb + kk) * RS + j0 + lr;
+        static_assert(BB % KC == 0, "whole products");
+        auto products = [&](auto edge_) {
+            constexpr bool edge = decltype(edge_)::value;   // some entries lie outside the band
 #pragma unroll
-                    for (int c = 0; c < TC; ++c) zc[c] = Z[(size_t)(sbb + u) * R + jq + RJ * c];
+            for (int u = 0; u < BB; u += KC) {
+                typename Tile::B b[NC];
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        const int d = rlo + rq + NQ * a - (cb + u);
-                        lv[a] = (sl[a] >= 0 && d <= mb) ? Lq[u * W + d] : Sc<T>::zero();
+                for (int c = 0; c < NC; ++c) b[c] = Tile::ldb(bp + u * RS + 8 * c);
+#pragma unroll
+                for (int a = 0; a < NR; ++a) {
+                    double av;
+                    if (edge) {
+                        const int over = max(0, d0 + a * step + lr - kk - u - mb);   // rows past the band: read its last entry
+                        av = Tile::lda_neg(ap[a] + u * (W - 1) - over);
+                        if (over) av = 0.0;
+                    } else {
+                        av = Tile::lda_neg(ap[a] + u * (W - 1));
                     }
 #pragma unroll
-                    for (int a = 0; a < 4; ++a)
-#pragma unroll
-                        for (int c = 0; c < TC; ++c) fms_acc(acc[a][c], lv[a], zc[c]);
+                    for (int c = 0; c < NC; ++c) acc[a][c].mma(av, b[c]);
                 }
             }
+        };
+        if (d0 + (NR - 1) * step + 7 <= mb) products(std::false_type{});
+        else products(std::true_type{});
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
-                if (sl[a] >= 0)
+        for (int a = 0; a < NR; ++a)
+            if (d0 + a * step + lr < dhi)
 #pragma unroll
-                    for (int c = 0; c < TC; ++c) Z[(size_t)sl[a] * R + jq + RJ * c] = acc[a][c];
-        }
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) zp[a][8 * c + q] = acc[a][c].get(q);
     };
-    issue_rows(start, min(n, start + BB + mb));
-    issue_rows(min(n, start + BB + mb), min(n, start + 2 * BB + mb));
-    fetch(start, 0);
-    if (start + BB < n) fetch(start + BB, 1);
-    cp_async_wait_group<1>();
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    // eight rows (slots from zh) of a block's triangle whose first column is
+    // Lh, for eight columns of the window: a lane per column, the other
+    // lanes repeat them
+    auto triangle = [&](auto wide_, const T* Lh, const T* dh, T* zh) {
+        constexpr bool wide = decltype(wide_)::value;   // mb >= 7: every entry is stored
+        auto l = [&](int t, int u) { return wide || t - u <= mb ? Lh[u * W + (t - u)] : Sc<T>::zero(); };
+        T* zc = zh + (lane & 7);
+        T z[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) z[t] = zc[(size_t)t * RS];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            z[u] = mul_fx(dh[u], z[u]);
+#pragma unroll
+            for (int t = u + 1; t < 8; ++t) fms_acc(z[t], l(t, u), z[u]);
+        }
+        if (lane < 8)
+#pragma unroll
+            for (int t = 0; t < 8; ++t) zc[(size_t)t * RS] = z[t];
+        __syncwarp();
+    };
+    for (int r = start + tid / R; r < min(n, start + BB + mb); r += NT / R) copy_row(tid % R, r, Z + (size_t)(r % WZ) * RS + tid % R);
+    cp_async_commit();
+    if (warp == FW) {
+        if (lane == 0) {
+            fetch(start, 0);
+            if (NB == 3 && start + BB < n) fetch(start + BB, 1);
+        }
+        __syncwarp();
+        pivots(0, 0, dinv[0]);
+    }
+    cp_async_wait_group<0>();
     __syncthreads();
-    int bi = 0;
+    int bi = 0, phs = 0, sc = start % WZ;   // sc: slot of the block's first row (WZ is a multiple of BB)
+    auto slot = [&](int d) { return sc + d < WZ ? sc + d : sc + d - WZ; };   // slot of row c0 + d, 0 <= d < WZ
     for (int c0 = start; c0 < n; c0 += BB, ++bi) {
-        const int nb = min(BB, n - c0);
-        const int cur = bi % 3, prv = (bi + 2) % 3;
-        wait(cur);
+        const int cur = bi % NB, prv = (bi + NB - 1) % NB, nxt = (bi + 1) % NB, sp = sc ? sc - BB : WZ - BB;
+        if (!mbar_wait(&bar[cur], phs >> cur & 1)) s_err = 1;
+        phs ^= 1 << cur;
         const T* Lc = Lb + (size_t)cur * BB * W;
         const T* Lp = Lb + (size_t)prv * BB * W;
-        if (tid < nb) dinv[tid] = Sc<T>::recip(Lc[tid * W]);
-        __syncthreads();
-        const int sb = c0 % WZ;
-        if (tid < 256) {
-            // A. block b's triangle: half-warp hw = column, lane lt = row
-            const int j = tid >> 4, lt = tid & 15;
-            const bool act = lt < nb;
-            T zt = Sc<T>::zero(), lrow[BB];
+        T* zb = Z + (size_t)sc * RS;
+        int node[NE];
+        double fk[NE];
+        if (warp < 2) {
+            // A. the triangle: rows 0-7, their products into rows 8-15, rows 8-15
+            T* zh = zb + 8 * warp;
+            auto tri = [&](const T* Lh, const T* dh, T* z) {
+                if (mb >= 7) triangle(std::true_type{}, Lh, dh, z);
+                else triangle(std::false_type{}, Lh, dh, z);
+            };
+            const T* di = dinv[bi & 1];
+            tri(Lc, di, zh);
+            {
+                Tile acc;
+                T* z8 = zh + (8 + lr) * RS + 2 * lg;
+                acc.set(0, z8[0]);
+                acc.set(1, z8[1]);
+                const int d0 = 8 + lr - Tile::kk();
+                const T* bp = zh + Tile::kk() * RS + lr;
+                const T* ap = Lc + Tile::kk() * W + d0;
 #pragma unroll
-            for (int u = 0; u < BB; ++u)
-                lrow[u] = (act && u < lt && lt - u <= mb) ? Lc[u * W + (lt - u)] : Sc<T>::zero();
-            if (act) zt = Z[(size_t)(sb + lt) * R + j];
+                for (int u = 0; u < 8; u += KC)
+                    {
+                    const int over = max(0, d0 - u - mb);
+                    const double av = Tile::lda_neg(ap + u * (W - 1) - over);
+                    acc.mma(over ? 0.0 : av, Tile::ldb(bp + u * RS));
+                }
+                z8[0] = acc.get(0);
+                z8[1] = acc.get(1);
+            }
+            __syncwarp();
+            tri(Lc + 8 * W, di + 8, zh + 8 * RS);
+        } else {
+            // A. the rows that block b + 1 needs start; block b - 1 into the
+            // rows [c0 + BB, c0 + mb); the next block's pivots
 #pragma unroll
-            for (int u = 0; u < BB; ++u) {
-                if (u < nb) {
-                    if (lt == u) zt = Sc<T>::mul(zt, dinv[u]);
-                    const T zu = shfl_w<T>(zt, u, 16);
-                    if (lt > u && lt < nb && lt - u <= mb) fms_acc(zt, lrow[u], zu);
+            for (int e = tid - 64; e < BB * R; e += 32 * NU) {
+                const int t = e % BB, r = c0 + BB + mb + t;
+                if (r < n) copy_row(e / BB, r, Z + (size_t)slot(BB + mb + t) * RS + e / BB);
+            }
+            cp_async_commit();
+            if (back && warp > FW)   // for phase B
+#pragma unroll
+                for (int q = 0; q < NE; ++q) {
+                    const int i = n - 1 - (c0 + (tid - 32 * (FW + 1) + q * OT) % BB);
+                    if (i >= 0) {
+                        node[q] = s.permI[i];
+                        fk[q] = fakws[(size_t)k * n + i];
+                    }
+                }
+            if (c0 > start) {
+                const int dhi = min(n - c0, mb);   // rows below c0
+                int d = BB + 8 * (warp - 2);
+                for (; d + 8 * NU < dhi; d += 16 * NU) {
+                    const int sr[2] = {slot(d), slot(d + 8 * NU)};
+                    update(I2{}, I2{}, Lp, sp, sr, d + BB, 8 * NU, dhi + BB, 0);
+                }
+                if (d < dhi) {
+                    const int sr[1] = {slot(d)};
+                    update(I1{}, I2{}, Lp, sp, sr, d + BB, 0, dhi + BB, 0);
                 }
             }
-            if (act) Z[(size_t)(sb + lt) * R + j] = zt;
-        } else if (c0 > start) {
-            // A. block b-1 (BB rows) into rows [c0 + BB, c0 + mb)
-            update_rows(Lp, c0 - BB, BB, min(n, c0 + BB), min(n, c0 + mb), 256, 256);
+            if (NB == 3 && warp == NT / 32 - 1 && c0 + BB < n) pivots(nxt, phs >> nxt & 1, dinv[bi + 1 & 1]);
+            cp_async_wait_group<1>();
         }
+        // block b-1's buffer is the destination of a copy below
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncthreads();
-        if (tid < 256) {
-            // B. block b's columns into block b+1's rows, an entry (row, column) per thread
-            const int j = tid & 15, t = tid >> 4, r = c0 + nb + t;
-            if (r < n && t < BB) {
-                T z = Z[(size_t)(r % WZ) * R + j];
-#pragma unroll
-                for (int u = 0; u < BB; ++u) {
-                    const int d = r - (c0 + u);
-                    if (u < nb && d <= mb) fms_acc(z, Lc[u * W + d], Z[(size_t)(sb + u) * R + j]);
-                }
-                Z[(size_t)(r % WZ) * R + j] = z;
-            }
+        if (warp < 4) {
+            // B. block b into block b+1's rows
+            const int d = BB + 8 * (warp >> 1), sr[1] = {slot(d)};
+            if (c0 + d < n) update(I1{}, I1{}, Lc, sc, sr, d, 0, min(n - c0, BB + mb), 8 * (warp & 1));
+        } else if (warp == FW) {
+            if (lane == 0 && c0 + (NB - 1) * BB < n) fetch(c0 + (NB - 1) * BB, prv);
+            __syncwarp();
+            if (NB == 2 && c0 + BB < n) pivots(nxt, phs >> nxt & 1, dinv[bi + 1 & 1]);
         } else {
             // B. block b's rows out
-            for (int idx = tid - 256; idx < nb * R; idx += 256) {
-                const int jj = idx / nb, t = idx % nb;
-                if (colid[jj] < 0) continue;
-                const int r = c0 + t;
-                const T v = Z[(size_t)(sb + t) * R + jj];
-                if (!back) {
-                    colp(jj)[r] = v;
-                } else {
-                    const int i = n - 1 - r;
-                    kpot[((size_t)k * s.L + colid[jj]) * n_kpot + s.permI[i]] =
-                        Sc<T>::to_cd(scale(v, fakws[(size_t)k * n + i]));
+#pragma unroll
+            for (int q = 0; q < NE; ++q) {
+                const int e = tid - 32 * (FW + 1) + q * OT, t = e % BB, j = e / BB;
+                if (j < R && c0 + t < n && colid[j] >= 0) {
+                    const T v = zb[(size_t)t * RS + j];
+                    if (!back) colp(j)[c0 + t] = v;
+                    else kpot[((size_t)k * s.L + colid[j]) * n_kpot + node[q]] = Sc<T>::to_cd(scale(v, fk[q]));
                 }
             }
         }
-        if (c0 + 2 * BB < n) fetch(c0 + 2 * BB, prv);
-        issue_rows(min(n, c0 + 2 * BB + mb), min(n, c0 + 3 * BB + mb));
-        cp_async_wait_group<1>();
         __syncthreads();
+        sc = sc + BB < WZ ? sc + BB : 0;
     }
     cp_async_wait_group<0>();
     if (tid == 0 && s_err) atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
@@ -1550,30 +1448,47 @@ __global__ void k_schur_out_gam(SchurArgs s, const T* __restrict__ xg, int n, cd
 
 // window rows: mb + 3 BB (the rows of a block, the band below it, and two
 // blocks arriving ahead), a multiple of BB
-int sweep_wz(int mbI) { return (mbI + 4 * SCHUR_MS_BB - 1) / SCHUR_MS_BB * SCHUR_MS_BB; }
+int sweep_wz(int mbI) { return (mbI + 4 * SW_BB - 1) / SW_BB * SW_BB; }
 
-constexpr int SWEEP_NT = 288;   // 4 x 4 update tiles of a 129-row band at R = 32 in one round
+}  // namespace
 
-// Columns per update tile of the sweeps: 2 (twice the threads, each with
-// half the accumulators) or 4.  Measured on the 60k-triangle mesh with the
-// half-warp triangles: back sweep and rebuild 20.6 ms with 2 against 24.0
-// with 4, the forward sweep's part after the factor 11.7 against 12.5;
-// CRT_B200_SCHUR_TILE=4 selects the wider tiles.
-static int sweep_tc(bool)
+// dynamic shared memory of a sweep with nb factor buffers
+template <typename T> static size_t sweep_smem(int mbI, int WI, int nb)
 {
-    const char* v = std::getenv("CRT_B200_SCHUR_TILE");
-    return (v && std::strcmp(v, "4") == 0) ? 4 : 2;
+    return ((size_t)nb * SW_BB * WI + (size_t)sweep_wz(mbI) * SweepRow<T>::v) * sizeof(T);
+}
+
+template <typename T> size_t schur_sweep_smem(int mbI, int WI) { return sweep_smem<T>(mbI, WI, 3); }
+
+namespace {
+
+// One launch of the sweep.  Launches of more CTAs than SMs pair two on an SM,
+// each with two factor buffers, while both fit (complex half-bandwidths to
+// 128): one's chain runs beside the other's updates.  Smaller ones give a CTA
+// its SM and three buffers, a block's pivots ahead of it.  Measured, paired
+// against alone: 128 sources and 492 boundary nodes at a half-bandwidth of
+// 128, the forward sweep's part after the factor (624 CTAs) 4.4 ms against
+// 6.5, the back sweep (128 CTAs) 6.3 against 4.7; 96 and 253 at 36, real, 0.02
+// against 0.23 (264 CTAs) and 0.75 against 0.50 (72).
+template <typename T>
+void sweep(const SchurArgs& s, int nblk, const T* Lws, const double* fakws, T* X, cd* kpot, int n_kpot, int back,
+           cudaStream_t st)
+{
+    constexpr int NT = 320;
+    const size_t two = sweep_smem<T>(s.mbI, s.WI, 2);
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const bool pair = (long long)s.nk * nblk > nsm && 2 * (two + 2048) <= 228 * 1024;
+    const size_t smem = pair ? two : schur_sweep_smem<T>(s.mbI, s.WI);
+    auto kern = pair ? k_schur_sweep<T, NT, 2, 2> : k_schur_sweep<T, NT, 3, 1>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<dim3(s.nk, nblk), NT, smem, st>>>(s, Lws, fakws, X, kpot, n_kpot, sweep_wz(s.mbI), back);
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
-template <typename T>
-size_t schur_sweep_smem(int mbI, int WI, int R)
-{
-    return (size_t)2 * SCHUR_MS_BB * WI * sizeof(T) + (size_t)sweep_wz(mbI) * R * sizeof(T);
-}
-
 template <typename T>
 void launch_schur_rhs(const SchurArgs& s, const BandArgs<T>& full, const double* fakws, T* X, T* cval, cudaStream_t st)
 {
@@ -1593,39 +1508,7 @@ void launch_schur_transpose(const SchurArgs& s, const T* Lws, T* Lrev, cudaStrea
 template <typename T>
 void launch_schur_forward(const SchurArgs& s, const T* Lws, T* X, cudaStream_t st)
 {
-    const size_t smem = schur_sweep_smem<T>(s.mbI, s.WI, s.R);
-    dim3 grid(s.nk, s.nblk);
-    auto go = [&](auto kern, int nt) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, nt, smem, st>>>(s, Lws, nullptr, X, nullptr, 0, sweep_wz(s.mbI), 0, 2);
-    };
-    // update tiles of 4 rows x TC columns: one round of a 129-row band
-    const bool narrow = sweep_tc(false) == 2;
-    const size_t smem_pp = (size_t)3 * SCHUR_MS_BB * s.WI * sizeof(T) + (size_t)sweep_wz(s.mbI) * 16 * sizeof(T);
-    const char* fv = std::getenv("CRT_B200_SCHUR_FWD");
-    if (s.R == 16 && fv && std::strcmp(fv, "pp") == 0 && smem_pp <= 227 * 1024) {
-        // 16-column blocks: the triangle beside the update (as the back sweep)
-        cudaFuncSetAttribute(k_schur_sweep_pp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_pp);
-        k_schur_sweep_pp<T><<<grid, 512, smem_pp, st>>>(s, Lws, nullptr, X, nullptr, 0, sweep_wz(s.mbI), 0);
-        return;
-    }
-    // 16-column blocks, rows one block ahead: the window of mb + 2 BB rows
-    // lets two CTAs share an SM (2 x 113 KB with the driver's reserve)
-    const int wz1 = (s.mbI + 2 * SCHUR_MS_BB + SCHUR_MS_BB - 1) / SCHUR_MS_BB * SCHUR_MS_BB;
-    const size_t smem1 = (size_t)2 * SCHUR_MS_BB * s.WI * sizeof(T) + (size_t)wz1 * 16 * sizeof(T);
-    if (s.R == 16 && !(fv && std::strcmp(fv, "wide") == 0) && 2 * (smem1 + 2048) <= 228 * 1024) {
-        auto kern = k_schur_sweep<T, 288, 16, SCHUR_MS_BB, 2, 2>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-        kern<<<grid, 288, smem1, st>>>(s, Lws, nullptr, X, nullptr, 0, wz1, 0, 1);
-        return;
-    }
-    if (s.R == 16) {
-        if (narrow) go(k_schur_sweep<T, 288, 16, SCHUR_MS_BB, 2>, 288);
-        else go(k_schur_sweep<T, 160, 16, SCHUR_MS_BB, 4>, 160);
-    } else {
-        if (narrow) go(k_schur_sweep<T, 544, SCHUR_MS_R, SCHUR_MS_BB, 2>, 544);
-        else go(k_schur_sweep<T, SWEEP_NT, SCHUR_MS_R, SCHUR_MS_BB, 4>, SWEEP_NT);
-    }
+    sweep<T>(s, s.nblk, Lws, nullptr, X, nullptr, 0, 0, st);
 }
 
 // One thread: returns once `want` CTAs of the concurrent factor have begun
@@ -1793,34 +1676,13 @@ template <typename T>
 void launch_schur_back(const SchurArgs& s, const T* Lrev, const double* fakws, const T* X, const T* xg, int n,
                        cd* kpot, cudaStream_t st)
 {
-    dim3 grid(s.nk, (s.L + SCHUR_BK_R - 1) / SCHUR_BK_R);
-    // the triangle beside the update (three factor buffers; 16.4 against
-    // 20.5 ms for back sweep and rebuild on the 60k-triangle mesh), unless
-    // CRT_B200_SCHUR_BACK_PP=0 or its buffers do not fit
-    const char* pv = std::getenv("CRT_B200_SCHUR_BACK_PP");
-    const size_t smem_pp = (size_t)3 * SCHUR_MS_BB * s.WI * sizeof(T) + (size_t)sweep_wz(s.mbI) * 16 * sizeof(T);
-    if (!(pv && std::strcmp(pv, "0") == 0) && smem_pp <= 227 * 1024) {
-        cudaFuncSetAttribute(k_schur_sweep_pp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_pp);
-        k_schur_sweep_pp<T><<<grid, 512, smem_pp, st>>>(s, Lrev, fakws, const_cast<T*>(X), kpot, n, sweep_wz(s.mbI), 1);
-        const long long tot = (long long)s.nk * s.L * s.m;
-        k_schur_out_gam<T><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s, xg, n, kpot);
-        return;
-    }
-    const size_t smem = schur_sweep_smem<T>(s.mbI, s.WI, SCHUR_BK_R);
-    auto go = [&](auto kern, int nt) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, nt, smem, st>>>(s, Lrev, fakws, const_cast<T*>(X), kpot, n, sweep_wz(s.mbI), 1, 2);
-    };
-    // 4 x 2 update tiles of a 129-row band at R = 16 in one round (288
-    // threads), or 4 x 4 (160)
-    if (sweep_tc(true) == 2) go(k_schur_sweep<T, 288, SCHUR_BK_R, SCHUR_MS_BB, 2>, 288);
-    else go(k_schur_sweep<T, 160, SCHUR_BK_R, SCHUR_MS_BB, 4>, 160);
+    sweep<T>(s, (s.L + SW_R - 1) / SW_R, Lrev, fakws, const_cast<T*>(X), kpot, n, 1, st);
     const long long tot = (long long)s.nk * s.L * s.m;
     k_schur_out_gam<T><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(s, xg, n, kpot);
 }
 
-template size_t schur_sweep_smem<cd>(int, int, int);
-template size_t schur_sweep_smem<double>(int, int, int);
+template size_t schur_sweep_smem<cd>(int, int);
+template size_t schur_sweep_smem<double>(int, int);
 template void launch_schur_rhs<cd>(const SchurArgs&, const BandArgs<cd>&, const double*, cd*, cd*, cudaStream_t);
 template void launch_schur_rhs<double>(const SchurArgs&, const BandArgs<double>&, const double*, double*, double*,
                                        cudaStream_t);

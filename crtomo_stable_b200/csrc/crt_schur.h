@@ -34,10 +34,8 @@
 
 // Largest boundary set the dense Schur kernels take (panel in shared memory).
 constexpr int SCHUR_MMAX = 768;
-// Columns per CTA of the forward sweep (all columns) and of the back sweep
-// (the source columns), and the row block of both.
-constexpr int SCHUR_MS_R = 32;
-constexpr int SCHUR_BK_R = 16;
+// Columns per CTA and row block of the sweeps.
+constexpr int SCHUR_MS_R = 16;
 constexpr int SCHUR_MS_BB = 16;
 
 // Host-side plan: node split, interior assembly lists, couplings.
@@ -62,7 +60,6 @@ struct SchurHost {
     // multi-RHS solve: columns ordered by their first non-zero interior
     // row; blocks of SCHUR_MS_R columns and their first rows
     std::vector<int> col_order, blk_start;
-    int R = SCHUR_MS_R;             // columns per block of the forward sweep (16 or 32)
     std::vector<int> first;         // [L + m] first non-zero interior row of each column
     std::vector<int> gsort, gfirst; // boundary positions by first row, and those rows
 };
@@ -72,13 +69,12 @@ struct SchurHost {
 // when the split is unusable (no interior or no boundary node, or m above
 // SCHUR_MMAX).
 int schur_plan_host(const AssemblyLists& full, int n, const std::vector<int>& gamma_nodes,
-                    const std::vector<int>& enr0, int lsink, int nsink0, SchurHost& out, int R = SCHUR_MS_R);
+                    const std::vector<int>& enr0, int lsink, int nsink0, SchurHost& out);
 
 // Device arguments of the Schur kernels (one context's plan).
 struct SchurArgs {
     int nI, m, L, K, ncol, mbI, WI, nblk, ncpl, ngg;
     int k0, nk;              // wavenumbers k0 .. k0 + nk - 1 of a launch (transpose .. back)
-    int R;                   // columns per block of the forward sweep (16: two CTAs per SM, 32: one)
     const int *permI, *gam, *posI_src, *posG_src;
     int posI_sink, posG_sink, lsink;
     const int *gi_ptr, *gi_pos, *gi_ent, *gi_g;
@@ -160,5 +156,5 @@ void launch_schur_zrebuild(const SchurArgs& s, T* X, const T* xg, cudaStream_t s
 template <typename T>
 void launch_schur_back(const SchurArgs& s, const T* Lrev, const double* fakws, const T* X, const T* xg, int n,
                        cd* kpot, cudaStream_t st);
-// Dynamic shared memory of a sweep for the interior band mbI with R columns.
-template <typename T> size_t schur_sweep_smem(int mbI, int WI, int R);
+// Dynamic shared memory of a sweep for the interior band mbI.
+template <typename T> size_t schur_sweep_smem(int mbI, int WI);

@@ -84,3 +84,25 @@ def test_boundary_systems(nx, nz, nel, ldc, solve, monkeypatch):
     kp_o = OracleProblem(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=kwnwi).forward(sigma, ldc=ldc, nthreads=8)
     assert np.abs(kp - kp_o).max() <= RTOL * np.abs(kp_o).max()
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,nz,nel", [(4, 2, 2), (9, 6, 4), (20, 7, 12), (18, 15, 9), (23, 16, 11), (40, 24, 17),
+                                       (30, 64, 9), (16, 121, 7), (16, 127, 7)])
+def test_sweeps_paired_or_alone(nx, nz, nel, monkeypatch):
+    """The triangular sweeps with two CTAs on an SM (launches of more CTAs
+    than SMs) and with one: a wavenumber's potentials are the same bit for bit
+    in a launch of 160 and alone, complex and real."""
+    from crtomo_stable_b200.lib import FORWARD_SCHUR, Context
+    monkeypatch.setenv("CRT_B200_SCHUR_SOLVE", "direct")
+    mesh, enr, strnr, vnr, sigma = survey(nx, nz, nel, True)
+    kwn = np.geomspace(0.01, 2.0, 160)
+    many = Context(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=np.ones(160))
+    one = Context(mesh, enr, strnr, vnr, kwn=kwn[77:78], kwnwi=np.ones(1))
+    for ldc in (False, True):
+        a = many.forward(sigma, ldc=ldc, want_kpot=True)[2]
+        assert many.forward_info()[0] == FORWARD_SCHUR
+        b = one.forward(sigma, ldc=ldc, want_kpot=True)[2]
+        assert np.array_equal(a[..., 77], b[..., 0])
+    many.close()
+    one.close()
