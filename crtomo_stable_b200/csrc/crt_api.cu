@@ -1419,12 +1419,11 @@ int jacobian_device(crt_ctx* ctx, int mode, const double* strom_h)
     S.part = ctx->d_part_sens;
     if (!ctx->d_sfac && !dalloc(ctx, &ctx->d_sfac, (size_t)ctx->N)) return CRT_ERR_ALLOC;
     S.rfac = ctx->d_sfac;
-    int LP = 0, gkc = 0, gnt = 0;
-    size_t gsmem = 0;
+    SensGram gram{};
     const char* sv = std::getenv("CRT_B200_SENS");
     const bool force_direct = sv && std::strcmp(sv, "direct") == 0;
-    if (!force_direct && sens_gram_plan(ctx->L, ctx->K, ctx->nkmax, real, &LP, &gkc, &gsmem, &gnt)) {
-        launch_sens_gram(S, LP, gkc, gsmem, gnt, real, ctx->st);
+    if (!force_direct && sens_gram_plan(ctx->L, ctx->K, ctx->nkmax, ctx->nmn, real, &gram)) {
+        launch_sens_gram(S, gram, real, ctx->st);
         ctx->launches += S.out_prec ? 2 : 1;
     } else {
         launch_sens(S, smem, real, ctx->st);

@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(NT) k_sens(SensArgs A)
 // wavenumbers (Phi_k and w_k E_k Phi_k), then written to shared memory for
 // the readings' gathers.
 constexpr int GR_TA = 4, GR_TB = 4;
+constexpr int SENS_KCMAX = 24;   // wavenumbers staged at once
 
 __device__ __forceinline__ int gram_idx(int a, int b)
 {
@@ -162,6 +163,190 @@ __device__ __forceinline__ int gram_idx(int a, int b)
     return a * (a + 1) / 2 + b;
 }
 
+// The readings of one element from its Gram matrix G (lower triangle, packed).
+template <typename T>
+__device__ __forceinline__ void gram_readings(const SensArgs& A, int e, const T* G)
+{
+    const int tid = threadIdx.x;
+    const cd sig = A.sigma[e];
+    // reading i: its four Gram entries, the reference's scaling, the store
+    auto value = [&](int4 el, int i) {
+        auto g = [&](int a, int b) { return (a < 0 || b < 0) ? Sc<T>::zero() : G[gram_idx(a, b)]; };
+        const T acc_i = ((g(el.w, el.y) - g(el.w, el.x)) - g(el.z, el.y)) + g(el.z, el.x);
+        cd res;
+        if (A.out_prec) {
+            // stored in FP32: each reading's divisions are done once
+            // (k_sens_factors), which changes the FP64 value only by
+            // rounding far below the stored precision
+            const cd f = A.rfac[i];
+            if (A.mode == 0) res = (Sc<T>::to_cd(acc_i) * f) * sig;
+            else if (A.mode == 1) res = cd{Sc<T>::to_cd(acc_i).x * (sig * f).x, 0.0};
+            else res = Sc<T>::to_cd(acc_i) * f.x;
+        } else if (A.mode == 0) {
+            // stored in FP64: the reference's operations in its order
+            cd d = Sc<T>::to_cd(acc_i);
+            if (A.swrtr != 0) d = d / A.pi;
+            res = (d * sig) / A.volt[i];
+        } else if (A.mode == 1) {
+            double d = Sc<T>::to_cd(acc_i).x;
+            if (A.swrtr != 0) d = d / A.pi;
+            const cd q = sig / A.volt[i];
+            res = cd{d * q.x, 0.0};
+        } else {
+            cd d = Sc<T>::to_cd(acc_i);
+            const double st = A.strom ? A.strom[i] : 1.0;
+            if (A.swrtr == 0) d = d * st;
+            else d = d * (st / A.pi);
+            res = -d;
+        }
+        return res;
+    };
+    auto store = [&](cd res, int i) {
+        const size_t o = (size_t)e * A.N + i;
+        if (A.mode == 1) {
+            if (A.out_prec) reinterpret_cast<float*>(A.sens)[o] = (float)res.x;
+            else reinterpret_cast<double*>(A.sens)[o] = res.x;
+        } else {
+            if (A.out_prec) reinterpret_cast<cf*>(A.sens)[o] = cf{(float)res.x, (float)res.y};
+            else reinterpret_cast<cd*>(A.sens)[o] = res;
+        }
+    };
+    // four readings per thread at a time: their (dependent) chains overlap
+    const int nt = blockDim.x;
+    for (int i0 = tid; i0 < A.N; i0 += 4 * nt) {
+        int4 el[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = i0 + q * nt;
+            el[q] = i < A.N ? A.elec[i] : make_int4(-1, -1, -1, -1);
+        }
+        cd res[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = i0 + q * nt;
+            res[q] = i < A.N ? value(el[q], i) : cd{0.0, 0.0};
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i0 + q * nt < A.N) store(res[q], i0 + q * nt);
+    }
+}
+
+// G on the FP64 tensor pipe, up to 128 electrodes (above, the accumulators of
+// the warps exceed the registers): a warp owns U units of 8 x 16 entries (row
+// block R, column blocks 2c and 2c + 1, those above the diagonal skipped) and
+// takes them over the staged rows q = (wavenumber, node) in ascending order by
+// m8n8k4 products, the factors of a complex product as two chains (fms_acc's
+// order).  Staged row stride LS = 4 mod 8, so the rows that a product's lanes
+// read together lie in different banks; rows are padded with zeros to whole
+// products.  A warp stages, and transforms by the element matrix (kept in
+// shared memory: read from global memory per entry it was 16,000 to 22,000
+// cycles of an element's time), whole rows.
+// Per element at 128 electrodes and 12,027 readings the readings' gathers are
+// 31,000 cycles, the products 27,000 on the FP64 pipe; one CTA's G fills an
+// SM, so the phases do not overlap.  60,160 triangles, 128 electrodes, 16
+// wavenumbers: 20.9 -> 17.2 ms; 8,000 triangles, 48 electrodes, 12
+// wavenumbers, 735 readings: 0.41 -> 0.31; real 0.31 -> 0.23; 704 rectangles,
+// 10 electrodes: 0.058 -> 0.025.
+template <typename T, int U, int MAXT>
+__global__ void __launch_bounds__(MAXT) k_sens_gram_mma(SensArgs A, int LS, int kc, int rows, int nunit)
+{
+    using Tile = MmaTile<T>;
+    constexpr int KC = Tile::KC;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int e = blockIdx.x;
+    const int nk = A.enk[e], nmn = A.nmn;
+    const int L = A.L, K = A.K;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = blockDim.x >> 5;
+    T* phi = reinterpret_cast<T*>(smem_raw);   // [rows][LS]
+    T* wu = phi + (size_t)rows * LS;           // [rows][LS]
+    __shared__ int s_node[4];
+    __shared__ double s_km[SENS_KCMAX * 10], s_w[SENS_KCMAX];
+    if (tid < nk) s_node[tid] = A.nrel0[e * A.maxnodes + tid];
+    Tile acc[U][2];
+    int ra[U], ca[U];   // the units' first rows and columns (ra < 0: none)
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+        const int u = warp + x * NW;
+        int R = 0, f = 0;   // units before row block R: f
+        while (f + R / 2 + 1 <= u) f += R++ / 2 + 1;
+        ra[x] = u < nunit ? 8 * R : -1;
+        ca[x] = 16 * (u - f);
+    }
+    const int lr = lane >> 2, lg = lane & 3, kk4 = Tile::kk();
+    for (int k0 = 0; k0 < K; k0 += kc) {
+        const int kn = min(kc, K - k0), nq = kn * nk, nq4 = (nq + 3) / 4 * 4;
+        __syncthreads();
+        // the potentials by cp.async (every copy of the thread in flight at
+        // once; the real form takes the real parts, 8 bytes each)
+        for (int q = warp; q < nq4; q += NW) {
+            T* dst = phi + (size_t)q * LS;
+            if (q < nq) {
+                const cd* src = A.kpt + ((size_t)(k0 + q / nk) * A.n + s_node[q % nk]) * L;
+                for (int a = lane; a < L; a += 32) phi_async<T>(dst + a, src + a);
+            } else {
+                for (int a = lane; a < LS; a += 32) dst[a] = wu[(size_t)q * LS + a] = Sc<T>::zero();
+            }
+        }
+        cp_async_commit();
+        for (int t = tid; t < kn * nmn; t += blockDim.x)
+            s_km[t] = A.elbg[((size_t)(k0 + t / nmn) * A.E + e) * nmn + t % nmn];
+        if (tid < kn) s_w[tid] = A.swrtr ? A.kwnwi[k0 + tid] : 1.0;
+        cp_async_wait_all();
+        __syncthreads();
+        for (int q = warp; q < nq; q += NW) {
+            const int kk = q / nk, m = q % nk;
+            const double w = s_w[kk];
+            double km[4];
+#pragma unroll
+            for (int m2 = 0; m2 < 4; ++m2) {
+                const int ix = max(m, m2), in = min(m, m2);
+                km[m2] = m2 < nk ? s_km[kk * nmn + ix * (ix + 1) / 2 + in] : 0.0;
+            }
+            const T* pr = phi + (size_t)kk * nk * LS;
+            T* dst = wu + (size_t)q * LS;
+            for (int b = lane; b < L; b += 32) {
+                T v = Sc<T>::zero();
+#pragma unroll
+                for (int m2 = 0; m2 < 4; ++m2)
+                    if (m2 < nk) v += scale(pr[(size_t)m2 * LS + b], km[m2]);
+                dst[b] = scale(v, w);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < U; ++x) {
+            if (ra[x] < 0) continue;
+            const T* pa = phi + (size_t)kk4 * LS + ra[x] + lr;
+            const T* pb = wu + (size_t)kk4 * LS + ca[x] + lr;
+            if (ca[x] + 8 <= ra[x]) {
+                for (int q = 0; q < nq; q += KC, pa += KC * LS, pb += KC * LS) {
+                    const typename Tile::A av = Tile::lda(pa);
+                    acc[x][0].mma(av, Tile::ldb(pb));
+                    acc[x][1].mma(av, Tile::ldb(pb + 8));
+                }
+            } else {
+                for (int q = 0; q < nq; q += KC, pa += KC * LS, pb += KC * LS) acc[x][0].mma(Tile::lda(pa), Tile::ldb(pb));
+            }
+        }
+    }
+    __syncthreads();
+    T* G = phi;   // lower triangle, packed
+#pragma unroll
+    for (int x = 0; x < U; ++x)
+        if (ra[x] >= 0)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int a = ra[x] + lr, b = ca[x] + 8 * c + 2 * lg + q;
+                    if (a >= b && a < L) G[a * (a + 1) / 2 + b] = acc[x][c].get(q);
+                }
+    __syncthreads();
+    gram_readings<T>(A, e, G);
+}
+
+// The same with a 4 x 4 tile of G per thread, above 128 electrodes.
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT) k_sens_gram(SensArgs A, int LP, int kc)
 {
@@ -273,68 +458,7 @@ __global__ void __launch_bounds__(MAXT) k_sens_gram(SensArgs A, int LP, int kc)
             }
     }
     __syncthreads();
-    const cd sig = A.sigma[e];
-    // reading i: its four Gram entries, the reference's scaling, the store
-    auto value = [&](int4 el, int i) {
-        auto g = [&](int a, int b) { return (a < 0 || b < 0) ? Sc<T>::zero() : G[gram_idx(a, b)]; };
-        const T acc_i = ((g(el.w, el.y) - g(el.w, el.x)) - g(el.z, el.y)) + g(el.z, el.x);
-        cd res;
-        if (A.out_prec) {
-            // stored in FP32: each reading's divisions are done once
-            // (k_sens_factors), which changes the FP64 value only by
-            // rounding far below the stored precision
-            const cd f = A.rfac[i];
-            if (A.mode == 0) res = (Sc<T>::to_cd(acc_i) * f) * sig;
-            else if (A.mode == 1) res = cd{Sc<T>::to_cd(acc_i).x * (sig * f).x, 0.0};
-            else res = Sc<T>::to_cd(acc_i) * f.x;
-        } else if (A.mode == 0) {
-            // stored in FP64: the reference's operations in its order
-            cd d = Sc<T>::to_cd(acc_i);
-            if (A.swrtr != 0) d = d / A.pi;
-            res = (d * sig) / A.volt[i];
-        } else if (A.mode == 1) {
-            double d = Sc<T>::to_cd(acc_i).x;
-            if (A.swrtr != 0) d = d / A.pi;
-            const cd q = sig / A.volt[i];
-            res = cd{d * q.x, 0.0};
-        } else {
-            cd d = Sc<T>::to_cd(acc_i);
-            const double st = A.strom ? A.strom[i] : 1.0;
-            if (A.swrtr == 0) d = d * st;
-            else d = d * (st / A.pi);
-            res = -d;
-        }
-        return res;
-    };
-    auto store = [&](cd res, int i) {
-        const size_t o = (size_t)e * A.N + i;
-        if (A.mode == 1) {
-            if (A.out_prec) reinterpret_cast<float*>(A.sens)[o] = (float)res.x;
-            else reinterpret_cast<double*>(A.sens)[o] = res.x;
-        } else {
-            if (A.out_prec) reinterpret_cast<cf*>(A.sens)[o] = cf{(float)res.x, (float)res.y};
-            else reinterpret_cast<cd*>(A.sens)[o] = res;
-        }
-    };
-    // four readings per thread at a time: their (dependent) chains overlap
-    const int nt = blockDim.x;
-    for (int i0 = tid; i0 < A.N; i0 += 4 * nt) {
-        int4 el[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = i0 + q * nt;
-            el[q] = i < A.N ? A.elec[i] : make_int4(-1, -1, -1, -1);
-        }
-        cd res[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = i0 + q * nt;
-            res[q] = i < A.N ? value(el[q], i) : cd{0.0, 0.0};
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (i0 + q * nt < A.N) store(res[q], i0 + q * nt);
-    }
+    gram_readings<T>(A, e, G);
 }
 
 // Each reading's factor of the Gram form's output for FP32 storage, so that
@@ -356,39 +480,73 @@ __global__ void k_sens_factors(SensArgs A)
     A.rfac[i] = f;
 }
 
-bool sens_gram_plan(int L, int K, int nkmax, bool real, int* LP_out, int* kc_out, size_t* smem_out, int* nt_out)
+bool sens_gram_plan(int L, int K, int nkmax, int nmn, bool real, SensGram* P)
 {
     const size_t tsz = real ? sizeof(double) : sizeof(cd);
     const int LP = (L + GR_TA - 1) / GR_TA * GR_TA;
     const int RB = LP / GR_TA, ntile = RB * (RB + 1) / 2;
     if (nkmax > 4 || ntile > 1024) return false;
+    P->mma = L <= 128 && nmn <= 10;
+    if (P->mma) {
+        const int RB8 = (L + 7) / 8;
+        const size_t gb = (size_t)L * (L + 1) / 2 * tsz;
+        P->LS = RB8 * 8 + 4;
+        auto bytes = [&](int kc) { return 2 * (size_t)((kc * nkmax + 3) / 4 * 4) * P->LS * tsz; };
+        int kc = std::min(K, SENS_KCMAX);
+        // staging no larger than G or 64 KB (48 electrodes: 0.31 ms, with 32 KB
+        // 0.29, with 96 KB 0.31; twelve streams' batch 15.05, 15.39, 15.11)
+        while (kc > 1 && bytes(kc) > std::max(gb, (size_t)64 * 1024)) --kc;
+        const int passes = (K + kc - 1) / kc;
+        P->kc = (K + passes - 1) / passes;
+        P->rows = (P->kc * nkmax + 3) / 4 * 4;
+        P->smem = std::max(gb, bytes(P->kc));
+        P->nunit = (RB8 / 2 + 1) * ((RB8 + 1) / 2);   // row block R has R / 2 + 1
+        // units per warp: few while the element has few (more warps share the
+        // staging and the gathers), five in 16 warps at 128 electrodes (72 units)
+        P->U = P->nunit <= 8 ? 1 : P->nunit <= 32 ? 2 : P->nunit <= 64 ? 4 : 5;
+        P->nt = 32 * (P->U == 5 ? 16 : std::max(4, (P->nunit + P->U - 1) / P->U));
+        return true;
+    }
     const size_t gbytes = (size_t)LP * (LP + 1) / 2 * tsz;
     const size_t limit = 200 * 1024;
     if (gbytes > limit) return false;
     int kc = K;
     while (kc > 1 && 2 * (size_t)kc * nkmax * LP * tsz > std::max(gbytes, (size_t)64 * 1024)) --kc;
-    *LP_out = LP;
-    *kc_out = kc;
-    *smem_out = std::max(gbytes, 2 * (size_t)kc * nkmax * LP * tsz);
-    *nt_out = (ntile + 31) / 32 * 32;
+    P->LS = LP;
+    P->kc = kc;
+    P->smem = std::max(gbytes, 2 * (size_t)kc * nkmax * LP * tsz);
+    P->nt = (ntile + 31) / 32 * 32;
     return true;
 }
 
-void launch_sens_gram(const SensArgs& a, int LP, int kc, size_t smem, int nt, bool real, cudaStream_t st)
+void launch_sens_gram(const SensArgs& a, const SensGram& P, bool real, cudaStream_t st)
 {
-    // one thread per tile: 320 threads up to 76 electrodes, 576 up to 132
     if (a.out_prec) k_sens_factors<<<(a.N + 255) / 256, 256, 0, st>>>(a);
+    if (P.mma) {
+        auto go = [&](auto kern) {
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem);
+            kern<<<a.E, P.nt, P.smem, st>>>(a, P.LS, P.kc, P.rows, P.nunit);
+        };
+        auto pick = [&](auto t) {
+            using T = decltype(t);
+            if (P.U == 1) go(k_sens_gram_mma<T, 1, 512>);
+            else if (P.U == 2) go(k_sens_gram_mma<T, 2, 512>);
+            else if (P.U == 4) go(k_sens_gram_mma<T, 4, 512>);
+            else go(k_sens_gram_mma<T, 5, 512>);
+        };
+        if (real) pick(double{});
+        else pick(cd{});
+        return;
+    }
     auto go = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<a.E, nt, smem, st>>>(a, LP, kc);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem);
+        kern<<<a.E, P.nt, P.smem, st>>>(a, P.LS, P.kc);
     };
     if (real) {
-        if (nt <= 320) go(k_sens_gram<double, 320>);
-        else if (nt <= 576) go(k_sens_gram<double, 576>);
+        if (P.nt <= 576) go(k_sens_gram<double, 576>);
         else go(k_sens_gram<double, 1024>);
     } else {
-        if (nt <= 320) go(k_sens_gram<cd, 320>);
-        else if (nt <= 576) go(k_sens_gram<cd, 576>);
+        if (P.nt <= 576) go(k_sens_gram<cd, 576>);
         else go(k_sens_gram<cd, 1024>);
     }
 }

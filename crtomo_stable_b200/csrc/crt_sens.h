@@ -29,5 +29,11 @@ void launch_sens(const SensArgs& a, size_t smem, bool real, cudaStream_t st);
 // Gram form (crt_sens.cu): false when the electrodes or element nodes
 // exceed its limits (L <= 168 for complex potentials, nk <= 4); then the
 // per-reading kernel above is used.
-bool sens_gram_plan(int L, int K, int nkmax, bool real, int* LP, int* kc, size_t* smem, int* nt);
-void launch_sens_gram(const SensArgs& a, int LP, int kc, size_t smem, int nt, bool real, cudaStream_t st);
+struct SensGram {
+    bool mma;              // on the FP64 tensor pipe
+    int LS, kc, nt;        // staged row stride, wavenumbers per pass, threads
+    int rows, nunit, U;    // tensor form: staged rows, units of G, units per warp
+    size_t smem;
+};
+bool sens_gram_plan(int L, int K, int nkmax, int nmn, bool real, SensGram* plan);
+void launch_sens_gram(const SensArgs& a, const SensGram& plan, bool real, cudaStream_t st);

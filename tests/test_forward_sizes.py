@@ -106,3 +106,30 @@ def test_sweeps_paired_or_alone(nx, nz, nel, monkeypatch):
         assert np.array_equal(a[..., 77], b[..., 0])
     many.close()
     one.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,nz,nel,tri", [(9, 3, 4, False), (14, 4, 8, True), (15, 4, 9, False), (24, 4, 16, True),
+                                           (25, 4, 17, False), (40, 3, 33, True), (55, 3, 48, False), (70, 3, 64, True),
+                                           (71, 3, 65, False), (120, 3, 113, True), (134, 3, 128, True),
+                                           (135, 3, 129, False)])
+def test_sensitivities_gram_against_direct(nx, nz, nel, tri, monkeypatch):
+    """The Gram form of the sensitivities at electrode counts where its tiles
+    and units have remainders (129: above the tensor form) against the
+    per-reading form.  A sum of 200 products rounds to 2e-14 of the largest;
+    the four-term combination leaves at least 1e-4 of it at a reading's
+    largest sensitivity, hence 1e-9 of that."""
+    from crtomo_stable_b200.lib import Context
+    mesh, enr, strnr, vnr, sigma = survey(nx, nz, nel, tri)
+    for mode in (0, 1, 2):
+        out = []
+        for kern in ("gram", "direct"):
+            if kern == "direct":
+                monkeypatch.setenv("CRT_B200_SENS", "direct")
+            else:
+                monkeypatch.delenv("CRT_B200_SENS", raising=False)
+            ctx = Context(mesh, enr, strnr, vnr)
+            ctx.forward(sigma, ldc=mode == 1)
+            out.append(ctx.jacobian(mode=mode))
+            ctx.close()
+        assert (np.abs(out[0] - out[1]) <= 1e-9 * np.abs(out[1]).max(axis=1, keepdims=True)).all()
