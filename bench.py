@@ -687,8 +687,8 @@ def main():
     if form_used == 2:
         w = schur_work(s, K, m_b, n_i, mb_i)
         it_mean = ph.get("schur_iter", 0.0)
-        chol_label = ("k_schur_chol (dense Cholesky of every S_l, fused forward solve, back solve)" if it_mean == 0 else
-                      "k_schur_s0 + k_schur_chol<REF> (a reference factor per 16 electrodes) + k_schur_iter "
+        chol_label = ("k_schur_ll (dense Cholesky of every S_l, fused forward solve, back solve)" if it_mean == 0 else
+                      "k_schur_s0 + k_schur_ll<REF> (a reference factor per 16 electrodes) + k_schur_iter "
                       "(preconditioned iteration per electrode, %.1f iterations)" % it_mean)
         if it_mean > 0:
             w["chol"] = w["chol_ref"] + it_mean * w["chol_it"]
@@ -699,7 +699,7 @@ def main():
         fwd_label = ("k_schur_sweep (forward sweep of [F r_I | F A_IG], beside the factor: span from the factor's "
                      "start) + factor transpose" if overlap else
                      "k_schur_sweep (forward sweep of [F r_I | F A_IG]) + factor transpose")
-        for name, key, label in (("factor", "factor_kernel", "k_band_factor_blk<cd> (interior band Cholesky, one system per wavenumber)"),
+        for name, key, label in (("factor", "factor_kernel", "k_band_factor_mma<cd> (interior band Cholesky, one system per wavenumber)"),
                                  ("forward", "schur_forward", fwd_label),
                                  ("gram", "schur_gram", "k_schur_gram (V^T [u^ | V^])"),
                                  ("chol", "schur_chol", chol_label),
