@@ -237,7 +237,11 @@ __global__ void k_schur_transpose(SchurArgs s, const T* __restrict__ Lws, T* Lre
 // column blocks).  The factor's columns stream through shared memory SW_BB at
 // a time (one bulk copy each, NB buffers, bounded mbarrier wait), the
 // right-hand sides live in a window Z of WZ rows (row r at slot r mod WZ, WZ
-// >= mb + 3 SW_BB), their rows arriving by cp.async two blocks ahead of use.
+// >= mb + 3 SW_BB), their rows arriving by cp.async: block b starts the copies
+// of rows c0 + 16 + mb .. c0 + 31 + mb.  Phase A of block b + 1 touches rows
+// below c0 + 16 + mb only where mb >= 16, so there they may still be in flight
+// when it begins; in narrower bands its triangle (rows c0 + 16 .. c0 + 31)
+// reaches them, and block b waits for its own copies (schur_sweep_in_flight).
 // Per block b (rows c0 .. c0 + 15), between barriers:
 //   A. warps 0 and 1 solve the block's triangle for eight columns each (a lane
 //      per column, 8 x 8 triangles in registers, the product between them on
@@ -287,7 +291,7 @@ template <> struct SweepTile<double> : MmaTile<double> {};
 template <typename T, int NT, int NB, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_schur_sweep(SchurArgs s, const T* __restrict__ Lws, const double* __restrict__ fakws, T* X, cd* kpot, int n_kpot,
-                  int WZ, int back)
+                  int WZ, int in_flight, int back)
 {
     constexpr int R = SW_R, BB = SW_BB, RS = SweepRow<T>::v;
     constexpr int NU = NT / 32 - 2;                              // update warps
@@ -515,7 +519,8 @@ __global__ void __launch_bounds__(NT, MINB)
                 }
             }
             if (NB == 3 && warp == NT / 32 - 1 && c0 + BB < n) pivots(nxt, phs >> nxt & 1, dinv[bi + 1 & 1]);
-            cp_async_wait_group<1>();
+            if (in_flight) cp_async_wait_group<1>();
+            else cp_async_wait_group<0>();
         }
         // block b-1's buffer is the destination of a copy below
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -1483,6 +1488,8 @@ template <typename T> static size_t sweep_smem(int mbI, int WI, int nb)
 
 template <typename T> size_t schur_sweep_smem(int mbI, int WI) { return sweep_smem<T>(mbI, WI, 3); }
 
+int schur_sweep_in_flight(int mbI) { return mbI >= SW_BB ? 1 : 0; }
+
 namespace {
 
 // One launch of the sweep.  Launches of more CTAs than SMs pair two on an SM,
@@ -1506,7 +1513,8 @@ void sweep(const SchurArgs& s, int nblk, const T* Lws, const double* fakws, T* X
     const size_t smem = pair ? two : schur_sweep_smem<T>(s.mbI, s.WI);
     auto kern = pair ? k_schur_sweep<T, NT, 2, 2> : k_schur_sweep<T, NT, 3, 1>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<dim3(s.nk, nblk), NT, smem, st>>>(s, Lws, fakws, X, kpot, n_kpot, sweep_wz(s.mbI), back);
+    kern<<<dim3(s.nk, nblk), NT, smem, st>>>(s, Lws, fakws, X, kpot, n_kpot, sweep_wz(s.mbI),
+                                            schur_sweep_in_flight(s.mbI), back);
 }
 
 }  // namespace

@@ -156,5 +156,8 @@ void launch_schur_zrebuild(const SchurArgs& s, T* X, const T* xg, cudaStream_t s
 template <typename T>
 void launch_schur_back(const SchurArgs& s, const T* Lrev, const double* fakws, const T* X, const T* xg, int n,
                        cd* kpot, cudaStream_t st);
+// Groups of row copies (the newest block's) that a sweep may leave in flight
+// when its next block begins.
+int schur_sweep_in_flight(int mbI);
 // Dynamic shared memory of a sweep for the interior band mbI.
 template <typename T> size_t schur_sweep_smem(int mbI, int WI);

@@ -133,3 +133,30 @@ def test_sensitivities_gram_against_direct(nx, nz, nel, tri, monkeypatch):
             out.append(ctx.jacobian(mode=mode))
             ctx.close()
         assert (np.abs(out[0] - out[1]) <= 1e-9 * np.abs(out[1]).max(axis=1, keepdims=True)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nz,tri", [(z, z % 2 == 1) for z in range(1, 19)])
+def test_sweeps_in_narrow_bands(nz, tri):
+    """Interior half-bandwidths of 1 to 18, below and above the sweeps'
+    blocks of 16 rows, over many blocks, two streams at once: the potentials
+    of the per-electrode band form, and the same bits from run to run."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from crtomo_stable_b200.lib import FORWARD_DIRECT, FORWARD_SCHUR, Context
+    mesh, enr, strnr, vnr, sigma = survey(150, nz, 12, tri)
+    kwn = np.geomspace(0.01, 2.0, 24)
+    ctxs = [Context(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=np.ones(24)) for _ in range(2)]
+    for ldc in (False, True):
+        def runs(ctx):
+            return [ctx.forward(sigma, ldc=ldc, want_kpot=True)[2] for _ in range(4)]
+        for c in ctxs:
+            c.set_forward_form(FORWARD_SCHUR)
+        with ThreadPoolExecutor(2) as ex:
+            first, *more = [kp for out in ex.map(runs, ctxs) for kp in out]
+        assert all(np.array_equal(first, kp) for kp in more)
+        ctxs[0].set_forward_form(FORWARD_DIRECT)
+        ref = runs(ctxs[0])[0]
+        assert np.abs(first - ref).max() <= RTOL * np.abs(ref).max()
+    for c in ctxs:
+        c.close()

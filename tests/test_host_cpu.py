@@ -156,3 +156,24 @@ def test_rcm_order_bandwidth_and_permutation():
     assert sorted(order) == [0, 1, 2, 3, 4] and bw == 1
     with pytest.raises(CRTError):
         rcm_order(np.array([0, 1]), np.array([5]))
+
+
+@pytest.mark.parametrize("mb", [1, 2, 7, 8, 10, 14, 15, 16, 17, 31, 32, 47, 128])
+def test_sweep_touches_no_row_in_flight(mb):
+    """The row copies of the Schur form's triangular sweep: a block of 16 rows
+    starts the copies of rows c0 + 16 + mb .. c0 + 31 + mb and leaves the
+    library's number of groups in flight; neither the triangle nor the updates
+    of any block touch a row whose copy has not been waited for."""
+    from crtomo_stable_b200 import lib
+    in_flight = lib.load()._Z21schur_sweep_in_flighti(mb)
+    groups = []
+    for c0 in range(0, 16 * 12, 16):
+        groups.append(range(c0 + 16 + mb, c0 + 32 + mb))
+        pending = {r for g in groups for r in g}
+        # phase A: the block's triangle, the block before into the rows past this block
+        assert pending.isdisjoint(range(c0, c0 + 16))
+        assert pending.isdisjoint(range(c0 + 16, c0 + mb))
+        groups = groups[len(groups) - in_flight:]
+        pending = {r for g in groups for r in g}
+        # phase B: the block into the next block's rows
+        assert pending.isdisjoint(range(c0 + 16, min(c0 + 32, c0 + 16 + mb)))
