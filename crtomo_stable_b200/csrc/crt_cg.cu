@@ -964,6 +964,9 @@ __global__ void __launch_bounds__(VS_UPD_NT) k_cg_tail_update(CGArgs A)
 // through its shared memory, and the vectors pass twice.  Against two sums
 // and two updates across the grid 14.6 us of kernels and three launches less
 // per iteration (9,600 cells).
+// A CTA may store into another's shared memory only once that CTA has begun:
+// every CTA arrives at a cluster barrier on entry and waits for it after
+// chain_wait, which hides its latency.
 constexpr int TURN_CTAS = 8, TURN_NT = VEC_NT / TURN_CTAS, TURN_UNROLL = 4;
 
 // the total of v over the cluster, in every thread; `slot` has a double per
@@ -980,8 +983,17 @@ __device__ __forceinline__ double cluster_total(double v, double* slot, int gwar
                      : "r"((unsigned)__cvta_generic_to_shared(slot + gwarp)), "r"(threadIdx.x & 31));
         asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(dst), "d"(v) : "memory");
     }
+    __syncwarp();   // the barrier is .aligned
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     return warp_allsum(slot[threadIdx.x & 31]);
+}
+
+// chain_wait of a cluster kernel; when it returns, the whole cluster has begun
+__device__ __forceinline__ void cluster_chain_wait()
+{
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+    chain_wait();
+    asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
 }
 
 __device__ void cg_turn_body(const CGArgs& A)
@@ -1042,7 +1054,7 @@ __device__ void cg_turn_body(const CGArgs& A)
 
 __global__ void __cluster_dims__(TURN_CTAS, 1, 1) __launch_bounds__(TURN_NT) k_cg_turn(CGArgs A)
 {
-    chain_wait();
+    cluster_chain_wait();
     cg_turn_body(A);
 }
 
@@ -1146,7 +1158,7 @@ __global__ void __launch_bounds__(VEC_NT) k_cgl_begin_pc(CGLArgs L) { cg_begin_p
 __global__ void __launch_bounds__(VEC_NT) k_cgl_end(CGLArgs L) { cg_end_body(cgl_cand(L, blockIdx.x)); }
 __global__ void __cluster_dims__(TURN_CTAS, 1, 1) __launch_bounds__(TURN_NT) k_cgl_turn(CGLArgs L)
 {
-    chain_wait();
+    cluster_chain_wait();
     cg_turn_body(cgl_cand(L, blockIdx.x / TURN_CTAS));
 }
 __global__ void __launch_bounds__(VEC_NT) k_cgl_finish(CGLArgs L, int lfpi, double step, const cd* par_in,

@@ -177,3 +177,24 @@ def test_sweep_touches_no_row_in_flight(mb):
         pending = {r for g in groups for r in g}
         # phase B: the block into the next block's rows
         assert pending.isdisjoint(range(c0 + 16, min(c0 + 32, c0 + 16 + mb)))
+
+
+def test_cluster_kernels_begin_with_a_cluster_barrier():
+    """A CTA may store into another's shared memory only once that CTA has
+    begun: every kernel with a cluster passes cluster_chain_wait (arrive on
+    entry, wait before anything else) first."""
+    import re
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = os.path.join(root, "crtomo_stable_b200", "csrc")
+    seen = 0
+    for name in sorted(os.listdir(src)):
+        with open(os.path.join(src, name)) as fh:
+            text = re.sub(r"//[^\n]*", "", fh.read())
+        for body in re.findall(r"__cluster_dims__[^{;]*\{([^}]*)\}", text):
+            assert re.match(r"\s*cluster_chain_wait\(\);", body), (name, body)
+            seen += 1
+        wait = re.search(r"void cluster_chain_wait\(\)\s*\{(.*?)\n\}", text, flags=re.S)
+        if wait:
+            steps = [wait.group(1).index(s) for s in ("barrier.cluster.arrive", "chain_wait();", "barrier.cluster.wait")]
+            assert steps == sorted(steps)
+    assert seen == 2
