@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(32 * (NU + 1), 1) k_band_factor_mma(BandArgs<T
             __syncthreads();
         }
     } else {
-        int P = 0;   // the panel's slot block
-        for (int i0 = 0, p = 0; !s_err; i0 += FP, ++p) {
+        int P = 0, p = 0;   // the panel's slot block, the panels taken
+        for (int i0 = 0; !s_err; i0 += FP, ++p) {
             const int Q = P + 1 == NB ? 0 : P + 1, inext = i0 + FP;
             fetch(inext + Wn, (p + 1) & 1);
             // ---- 1. rows below the panel, four columns at a time
@@ -321,6 +321,13 @@ __global__ void __launch_bounds__(32 * (NU + 1), 1) k_band_factor_mma(BandArgs<T
             P = Q;
             __syncthreads();
         }
+        // Copy c (rows Wn + 8 c on) is awaited by panel c, a panel after its
+        // start: when a pivot ends the loop with p panels taken, copy p is in
+        // flight (and p - 1, if its wait gave up).  The CTA's shared memory
+        // must not be left to it.
+        if (tid == NT - 1 && s_err)
+            for (int c = max(0, p - 1); c <= p; ++c)
+                if (Wn + FP * c < n) mbar_wait(&bar[c & 1], (c >> 1) & 1);
     }
     __syncthreads();
     if (tid == 0 && s_err) A.status[sys] = s_err;

@@ -160,3 +160,24 @@ def test_sweeps_in_narrow_bands(nz, tri):
         assert np.abs(first - ref).max() <= RTOL * np.abs(ref).max()
     for c in ctxs:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("col", [1, 2, 3, 17, 30, 44, 57, 58])
+def test_pivot_breakdown_in_registers(col):
+    """A negative cell makes the interior system indefinite at its column of
+    the mesh (early, middle and last panels of the factor): an error, and the
+    next forward on the context gives the bits of the one before."""
+    from crtomo_stable_b200.lib import CRTError, FORWARD_SCHUR, Context
+    mesh, enr, strnr, vnr, _ = survey(60, 20, 9, False)
+    sigma = np.full(mesh.elanz, 0.01, np.complex128)
+    ctx = Context(mesh, enr, strnr, vnr)
+    kp = ctx.forward(sigma, ldc=True, want_kpot=True)[2]
+    assert ctx.forward_info()[0] == FORWARD_SCHUR
+    bad = sigma.copy()
+    bad[8 * 60 + col] = -0.02
+    for _ in range(3):
+        with pytest.raises(CRTError):
+            ctx.forward(bad, ldc=True)
+        assert np.array_equal(ctx.forward(sigma, ldc=True, want_kpot=True)[2], kp)
+    ctx.close()
