@@ -328,7 +328,8 @@ __global__ void __launch_bounds__(NT, MINB)
             // the factor's columns [c0, c0 + BB) are final once its
             // progress passes them.  The wait gives up after about 4 s,
             // or at once when another CTA of this wavenumber gave up
-            // (status set); the result is then flagged as failed.
+            // (status set); the result is then flagged as failed, and an
+            // error that the factor recorded stays.
             const int want = min(n, c0 + BB);
             long polls = 0;
             int got;
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(NT, MINB)
                 if (got >= want) break;
                 if (*(volatile const int*)(s.status + k) != 0 || ++polls > (1L << 22)) {
                     s_err = 1;
-                    atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
+                    atomicCAS(&s.status[k], 0, (int)CRT_ERR_CUDA);
                     break;
                 }
                 __nanosleep(256);
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(NT, MINB)
         sc = sc + BB < WZ ? sc + BB : 0;
     }
     cp_async_wait_group<0>();
-    if (tid == 0 && s_err) atomicMax(&s.status[k], (int)CRT_ERR_CUDA);
+    if (tid == 0 && s_err) atomicCAS(&s.status[k], 0, (int)CRT_ERR_CUDA);
 }
 
 // ---------------------------------------------------------------------------

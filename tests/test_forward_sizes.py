@@ -181,3 +181,20 @@ def test_pivot_breakdown_in_registers(col):
             ctx.forward(bad, ldc=True)
         assert np.array_equal(ctx.forward(sigma, ldc=True, want_kpot=True)[2], kp)
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("col", [1, 30, 57])
+def test_factor_error_is_reported(col):
+    """A pivot that breaks down is error 28, whether or not the sweep beside
+    the factor notices first."""
+    from crtomo_stable_b200.lib import CRTError, Context
+    mesh, enr, strnr, vnr, _ = survey(60, 20, 9, False)
+    sigma = np.full(mesh.elanz, 0.01, np.complex128)
+    sigma[8 * 60 + col] = -0.02
+    ctx = Context(mesh, enr, strnr, vnr)
+    for _ in range(5):
+        with pytest.raises(CRTError) as ei:
+            ctx.forward(sigma, ldc=True)
+        assert ei.value.errnr == 28
+    ctx.close()
