@@ -1742,7 +1742,7 @@ int update_device(crt_ctx* ctx, const crt_cg_params* prm, const cd* d_sigmaa, in
     ctx->cg_form = use_block ? (use_gnn ? CRT_PRECOND_BLOCK_GNN : CRT_PRECOND_BLOCK)
                              : (use_gnn ? CRT_PRECOND_GNN : CRT_PRECOND_JACOBI);
     if (int e = setup_cg_fused(ctx, &a)) return e;
-    a.turn = !a.pc;
+    a.turn = !a.pc && a.M <= CG_TURN_MAX;
     launch_cg_init(a, ctx->st);
     ctx->launches += a.turn ? 3 : 1;
     CK(cudaEventRecord(ctx->ev[1], ctx->st));

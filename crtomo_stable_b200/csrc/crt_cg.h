@@ -19,6 +19,14 @@ struct CGState {
     int vcnt, pending, ucnt, use_base;
 };
 
+// Most cells for which one cluster ends an iteration and begins the next: its
+// 1,024 threads pass over the vectors, which costs less than three launches
+// only while they are short.  An iteration with it and by the grid-wide
+// kernels (the same sums, bit for bit): 2,400 cells 18.2 and 26.6 us, 9,600
+// 36.7 and 43.5, 14,400 33.3 and 38.2, 24,000 57.8 and 57.5, 36,000 92.1 and
+// 90.8, 60,160 99.9 and 93.5, 120,000 235 and 210.
+constexpr int CG_TURN_MAX = 24 * 1024;
+
 struct CGArgs {
     int M, N;             // manz, nanz
     int jmode;            // 0 complex J (cjggra), 1 real sensdc (ldc), 2 real part of complex J (lfpi)
@@ -56,9 +64,9 @@ struct CGArgs {
     unsigned long long* fepoch;   // [1] advanced by every iteration tail (tickets stay unique)
     int* ferr;                    // [1] set when a wait gave up
     int flag_lag;                 // row blocks between a block's two uses (CGF_S .. CGF_Q - 1)
-    // Jacobi form: one kernel ends an iteration and begins the next
-    // (k_cg_turn; the first head runs with launch_cg_init), instead of a tail
-    // and a head of two kernels each
+    // Jacobi form up to CG_TURN_MAX cells: one kernel ends an iteration and
+    // begins the next (k_cg_turn; the first head runs with launch_cg_init),
+    // instead of a tail and a head of two kernels each
     int turn;
     double* vred;                 // [32][8] per-CTA partial sums of the grid-wide head and tail
 };

@@ -44,3 +44,11 @@ def test_update_and_lambda_candidates(nx, nz, nel, ldc):
     lam0 = float(5.0 * np.abs(J.conj().T @ (wd * J.sum(1))).sum() / M)
     assert abs(ctx.blam0(1.0, 1.0, ldc=ldc) - lam0) <= 1e-12 * lam0
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,nz", [(192, 128), (220, 112)])
+def test_update_where_the_turns_end(nx, nz):
+    """24,576 cells, the most that one cluster turns an iteration over for, and
+    24,640, by the grid-wide kernels."""
+    test_update_and_lambda_candidates(nx, nz, 6, False)
