@@ -15,7 +15,7 @@
 //   k_schur_ll      per (k, l): S_l = A_GG(l) - V^T V^, left-looking blocked
 //       Cholesky (unconjugated, complex symmetric as src/chol.f90:44-78), the
 //       forward solve fused into the factorisation, the back solve by panels
-//       (k_schur_chol, right-looking, for the largest complex boundaries);
+//       (k_schur_chol, right-looking, for the larger boundaries: ll_staged);
 //   k_schur_zrebuild  z^ = u^ - V^ p_G (tiled GEMM);
 //   k_schur_out_gam p_G into kpot at the boundary nodes.
 #include "crt_schur.h"
@@ -1475,6 +1475,14 @@ __global__ void k_schur_out_gam(SchurArgs s, const T* __restrict__ xg, int n, cd
     kpot[kl * n + s.gam[g]] = Sc<T>::to_cd(xg[kl * s.m + g]);
 }
 
+int sm_count()
+{
+    int nsm = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
 // window rows: mb + 3 BB (the rows of a block, the band below it, and two
 // blocks arriving ahead), a multiple of BB
 int sweep_wz(int mbI) { return (mbI + 4 * SW_BB - 1) / SW_BB * SW_BB; }
@@ -1507,10 +1515,7 @@ void sweep(const SchurArgs& s, int nblk, const T* Lws, const double* fakws, T* X
 {
     constexpr int NT = 320;
     const size_t two = sweep_smem<T>(s.mbI, s.WI, 2);
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const bool pair = (long long)s.nk * nblk > nsm && 2 * (two + 2048) <= 228 * 1024;
+    const bool pair = (long long)s.nk * nblk > sm_count() && 2 * (two + 2048) <= 228 * 1024;
     const size_t smem = pair ? two : schur_sweep_smem<T>(s.mbI, s.WI);
     auto kern = pair ? k_schur_sweep<T, NT, 2, 2> : k_schur_sweep<T, NT, 3, 1>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1577,10 +1582,7 @@ void launch_schur_gram(const SchurArgs& s, const T* X, T* C, cudaStream_t st)
     // lose on every size (60k triangles: 12.5 ms at 64 x 64, 10.8 at 64 x 32):
     // a tile runs from the earliest row of its columns, and its serial sum
     // over the rows is the longest CTA's time.
-    int nsm = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if ((long long)s.nk * ((s.m + 31) / 32) * ((s.ncol + 31) / 32) >= 5 * nsm)
+    if ((long long)s.nk * ((s.m + 31) / 32) * ((s.ncol + 31) / 32) >= 5 * sm_count())
         go(k_schur_gram<T, 32, 32, 2, 2, 4>, 32, 32, 128, 4);
     else
         go(k_schur_gram<T, 32, 16, 2, 1, 4>, 32, 16, 128, 4);
@@ -1590,6 +1592,23 @@ void launch_schur_gram(const SchurArgs& s, const T* X, T* C, cudaStream_t st)
 // above 553 complex boundary nodes
 template <typename T>
 static int ll_back_panel(int m) { return 2 * ((size_t)13 * m * sizeof(T) + 1024) <= 227 * 1024 ? 12 : 16; }
+
+// Whether nsys systems of m boundary nodes go left-looking with their stages
+// in shared memory: always while two such CTAs share an SM (complex to 256
+// nodes, real to 488), and above only where every system has an SM of its
+// own, up to a size at which the right-looking form's two CTAs win even there.
+// Left and right in ms, complex: 1,152 systems of 241 nodes 3.95 and 4.57, of
+// 261 6.48 and 5.26, of 401 18.9 and 13.4; 140 of 361 1.84 and 1.96, of 401
+// 2.42 and 2.45, of 481 3.88 and 3.72.  Real: 1,152 of 481 10.3 and 12.0, of
+// 521 16.1 and 14.5, of 767 61 and 41; 140 of 601 3.53 and 3.78, of 701 5.57
+// and 5.42.  The two give the same bits.
+template <typename T>
+static bool ll_staged(int m, int nsys)
+{
+    const size_t smem = ll_smem<T>(m, false), cta = 2560;   // a CTA's static shared memory and the driver's share
+    if (2 * (smem + cta) <= 228 * 1024) return true;
+    return nsys <= sm_count() && m <= (std::is_same<T, cd>::value ? 400 : 640);
+}
 
 template <typename T>
 void launch_schur_chol(const SchurArgs& s, const BandArgs<T>& full, const T* C, T* Sws, T* xg, int sys0, int nsys,
@@ -1607,19 +1626,19 @@ void launch_schur_chol(const SchurArgs& s, const BandArgs<T>& full, const T* C, 
         go(k_schur_ll<T, true, false, LL_NT, 4>, ll_smem<T>(s.m, true));
         return;
     }
-    if (ll_smem<T>(s.m, false) <= lim) {
+    if (ll_staged<T>(s.m, nsys)) {
         go(k_schur_ll<T, false, false, LL_NT, 4>, ll_smem<T>(s.m, false));
         return;
     }
-    // above 536 complex boundary nodes the stages do not fit: right-looking,
-    // two CTAs per SM with 12-column panels up to 553, else one with 16
+    // right-looking: two CTAs per SM with 12-column panels up to 553 complex
+    // boundary nodes, else one with 16
     constexpr int NT = 256;
     const size_t smem16 = ((size_t)16 * s.m + s.m) * sizeof(T), smem12 = ((size_t)12 * s.m + s.m) * sizeof(T);
     if (ll_back_panel<T>(s.m) == 12) {
         auto kern = k_schur_chol<T, NT, 12, false>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem12);
         kern<<<nsys, NT, smem12, st>>>(s, full, C, Sws, xg, sys0, nullptr);
-    } else {
+    } else if constexpr (std::is_same<T, cd>::value) {   // real: SCHUR_MMAX nodes take 12
         auto kern = k_schur_chol<T, NT, 16, true>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem16);
         kern<<<nsys, NT, smem16, st>>>(s, full, C, Sws, xg, sys0, nullptr);
@@ -1640,7 +1659,12 @@ void launch_schur_ref(const SchurArgs& s, const BandArgs<T>& full, const T* S0, 
 {
     const int nref = s.K * s.ngrp;
     const size_t smem = ll_smem<T>(s.m, false);
-    if (smem <= 227 * 1024) {
+    // left-looking with 512 threads on an SM while its stages fit (complex to
+    // 528 boundary nodes) and every factor has an SM (complex, 128 of 492: 3.0
+    // ms against 3.4 right-looking, but 300 of 441 0.5 longer); real up to 640
+    // nodes at any number (300 of 521 1.1 shorter, 450 of 761 2.2 longer)
+    const bool real = std::is_same<T, double>::value;
+    if (smem <= 227 * 1024 && (nref <= sm_count() || (real && s.m <= 640))) {
         auto kern = k_schur_ll<T, false, true, 512, 4>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<nref, 512, smem, st>>>(s, full, S0, Lref, nullptr, 0, 0, nonconv);
@@ -1652,7 +1676,7 @@ void launch_schur_ref(const SchurArgs& s, const BandArgs<T>& full, const T* S0, 
         auto kern = k_schur_chol<T, NT, 12, false, true>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem12);
         kern<<<nref, NT, smem12, st>>>(s, full, S0, Lref, nullptr, 0, nonconv);
-    } else {
+    } else if constexpr (std::is_same<T, cd>::value) {   // real: SCHUR_MMAX nodes take 12
         auto kern = k_schur_chol<T, NT, 16, true, true>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem16);
         kern<<<nref, NT, smem16, st>>>(s, full, S0, Lref, nullptr, 0, nonconv);

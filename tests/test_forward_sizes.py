@@ -198,3 +198,25 @@ def test_factor_error_is_reported(col):
             ctx.forward(sigma, ldc=True)
         assert ei.value.errnr == 28
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solve", ["direct", "iter"])
+@pytest.mark.parametrize("nodes", [255, 256, 257, 399, 401, 488, 489, 527, 529, 641, 767])
+def test_boundary_systems_of_many_or_few(nodes, solve, monkeypatch):
+    """The boundary systems (or reference factors) of 160 wavenumbers, more
+    than SMs, and of one wavenumber, at both sides of where the left-looking
+    factor takes over from the right-looking one: the same bits."""
+    from crtomo_stable_b200.lib import FORWARD_SCHUR, Context
+    monkeypatch.setenv("CRT_B200_SCHUR_SOLVE", solve)
+    mesh, enr, strnr, vnr, sigma = survey(nodes - 17, 8, 2, False)
+    kwn = np.geomspace(0.01, 2.0, 160)
+    many = Context(mesh, enr, strnr, vnr, kwn=kwn, kwnwi=np.ones(160))
+    one = Context(mesh, enr, strnr, vnr, kwn=kwn[77:78], kwnwi=np.ones(1))
+    for ldc in (False, True):
+        a = many.forward(sigma, ldc=ldc, want_kpot=True)[2]
+        assert many.forward_info()[:2] == (FORWARD_SCHUR, nodes)
+        b = one.forward(sigma, ldc=ldc, want_kpot=True)[2]
+        assert np.array_equal(a[..., 77], b[..., 0])
+    many.close()
+    one.close()
