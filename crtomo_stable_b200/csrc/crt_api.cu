@@ -1422,7 +1422,7 @@ int jacobian_device(crt_ctx* ctx, int mode, const double* strom_h)
     SensGram gram{};
     const char* sv = std::getenv("CRT_B200_SENS");
     const bool force_direct = sv && std::strcmp(sv, "direct") == 0;
-    if (!force_direct && sens_gram_plan(ctx->L, ctx->K, ctx->nkmax, ctx->nmn, real, &gram)) {
+    if (!force_direct && sens_gram_plan(ctx->L, ctx->E, ctx->K, ctx->nkmax, ctx->nmn, real, &gram)) {
         launch_sens_gram(S, gram, real, ctx->st);
         ctx->launches += S.out_prec ? 2 : 1;
     } else {

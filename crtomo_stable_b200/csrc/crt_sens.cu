@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(MAXT) k_sens_gram_mma(SensArgs A, int LS, int 
     gram_readings<T>(A, e, G);
 }
 
-// The same with a 4 x 4 tile of G per thread, above 128 electrodes.
+// The same with a 4 x 4 tile of G per thread, above 128 electrodes and where
+// sens_gram_plan says so.
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT) k_sens_gram(SensArgs A, int LP, int kc)
 {
@@ -480,13 +481,21 @@ __global__ void k_sens_factors(SensArgs A)
     A.rfac[i] = f;
 }
 
-bool sens_gram_plan(int L, int K, int nkmax, int nmn, bool real, SensGram* P)
+bool sens_gram_plan(int L, int E, int K, int nkmax, int nmn, bool real, SensGram* P)
 {
     const size_t tsz = real ? sizeof(double) : sizeof(cd);
     const int LP = (L + GR_TA - 1) / GR_TA * GR_TA;
     const int RB = LP / GR_TA, ntile = RB * (RB + 1) / 2;
     if (nkmax > 4 || ntile > 1024) return false;
-    P->mma = L <= 128 && nmn <= 10;
+    // Not on the tensor pipe: few electrodes on many elements (above about
+    // eight an SM), where a CTA of four warps spends its time on padding and
+    // barriers (real, 10 electrodes, 25,600 elements: 0.24 ms against 0.15,
+    // 16: 0.29 against 0.20; complex, 8: 0.25 against 0.21; 300 elements the
+    // other way by a tenth), and real ones of 81 to 96 electrodes, whose 36 to
+    // 42 units make 9 to 11 warps of four and leave room for one CTA an SM (96:
+    // 2.04 against 1.80; 80: 1.25 against 1.77, 98: 2.19 against 2.84).
+    const bool few = L <= (real ? 16 : 8) && E > 8 * 148;
+    P->mma = L <= 128 && nmn <= 10 && !few && !(real && L > 80 && L <= 96);
     if (P->mma) {
         const int RB8 = (L + 7) / 8;
         const size_t gb = (size_t)L * (L + 1) / 2 * tsz;
@@ -502,8 +511,12 @@ bool sens_gram_plan(int L, int K, int nkmax, int nmn, bool real, SensGram* P)
         P->smem = std::max(gb, bytes(P->kc));
         P->nunit = (RB8 / 2 + 1) * ((RB8 + 1) / 2);   // row block R has R / 2 + 1
         // units per warp: few while the element has few (more warps share the
-        // staging and the gathers), five in 16 warps at 128 electrodes (72 units)
-        P->U = P->nunit <= 8 ? 1 : P->nunit <= 32 ? 2 : P->nunit <= 64 ? 4 : 5;
+        // staging and the gathers), five in 16 warps at 128 electrodes (72
+        // units); four from where warps of two leave an SM to one CTA (25,600
+        // elements, two and four: complex, 64 electrodes 1.36 and 1.36 ms, 66
+        // 2.49 and 1.82, 80 2.72 and 2.01; real, 72 0.95 and 1.29, 74 1.58 and
+        // 1.22)
+        P->U = P->nunit <= 8 ? 1 : P->nunit <= (real ? 25 : 20) ? 2 : P->nunit <= 64 ? 4 : 5;
         P->nt = 32 * (P->U == 5 ? 16 : std::max(4, (P->nunit + P->U - 1) / P->U));
         return true;
     }
@@ -543,10 +556,12 @@ void launch_sens_gram(const SensArgs& a, const SensGram& P, bool real, cudaStrea
         kern<<<a.E, P.nt, P.smem, st>>>(a, P.LS, P.kc);
     };
     if (real) {
-        if (P.nt <= 576) go(k_sens_gram<double, 576>);
+        if (P.nt <= 320) go(k_sens_gram<double, 320>);
+        else if (P.nt <= 576) go(k_sens_gram<double, 576>);
         else go(k_sens_gram<double, 1024>);
     } else {
-        if (P.nt <= 576) go(k_sens_gram<cd, 576>);
+        if (P.nt <= 320) go(k_sens_gram<cd, 320>);
+        else if (P.nt <= 576) go(k_sens_gram<cd, 576>);
         else go(k_sens_gram<cd, 1024>);
     }
 }

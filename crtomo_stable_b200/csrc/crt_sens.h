@@ -35,5 +35,5 @@ struct SensGram {
     int rows, nunit, U;    // tensor form: staged rows, units of G, units per warp
     size_t smem;
 };
-bool sens_gram_plan(int L, int K, int nkmax, int nmn, bool real, SensGram* plan);
+bool sens_gram_plan(int L, int E, int K, int nkmax, int nmn, bool real, SensGram* plan);
 void launch_sens_gram(const SensArgs& a, const SensGram& plan, bool real, cudaStream_t st);

@@ -220,3 +220,15 @@ def test_boundary_systems_of_many_or_few(nodes, solve, monkeypatch):
         assert np.array_equal(a[..., 77], b[..., 0])
     many.close()
     one.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,nz,nel,tri", [(149, 8, 8, False), (148, 8, 8, False), (80, 8, 9, True), (80, 8, 16, True),
+                                           (80, 8, 17, True), (110, 3, 72, True), (110, 3, 73, False),
+                                           (110, 3, 80, True), (110, 3, 81, False), (110, 3, 96, True),
+                                           (110, 3, 97, False)])
+def test_sensitivities_where_the_gram_form_changes(nx, nz, nel, tri, monkeypatch):
+    """Electrode and element counts at both sides of where the Gram form takes
+    another kernel or another number of units per warp, as in
+    test_sensitivities_gram_against_direct."""
+    test_sensitivities_gram_against_direct(nx, nz, nel, tri, monkeypatch)
