@@ -110,7 +110,7 @@ struct crt_ctx {
     CGState* d_live = nullptr;   // a never-done CG state for preconditioner applications outside the CG
     double* d_vred = nullptr;    // partial sums of the CG head and tail
     cd* d_sfac = nullptr;        // per-reading factors of the Gram-form Jacobian
-    double* d_colsum = nullptr;  // sums over the Jacobian's columns and readings (lambda_0, coverage), kept
+    double* d_colsum = nullptr;  // sums over a set Jacobian's columns and readings (lambda_0, coverage), kept
     // the forward sweep concurrent with the interior factor: the factor's
     // progress per wavenumber and its count of started CTAs, the stream and
     // the fork / join events
@@ -1875,13 +1875,19 @@ __global__ void k_coverage_col(const S* __restrict__ J, int N, int M, int re_par
     if (lane == 0) csens[j] = acc;
 }
 
-// Readings' sums (blam0) or weights (coverage), then a double per cell: one
-// buffer, allocated at the first call (an allocation and a release per call
-// cost up to milliseconds)
-int ensure_colsum(crt_ctx* ctx)
+// Readings' sums (blam0) or weights (coverage), then a double per cell, in the
+// transposed potentials, which only the Jacobian's own pass reads, where they
+// are long enough; else in a buffer allocated at the first call (for a
+// Jacobian that the caller set).  With a buffer the first lambda_0 and
+// coverage of a context took 0.50 ms, the later ones 0.14.
+int colsum_space(crt_ctx* ctx, double** ws)
 {
-    if (ctx->d_colsum) return CRT_OK;
-    return dalloc(ctx, &ctx->d_colsum, 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT) + (size_t)ctx->E) ? CRT_OK : CRT_ERR_CUDA;
+    const size_t need = 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT) + (size_t)ctx->E;
+    *ws = reinterpret_cast<double*>(ctx->d_kpt);
+    if (ctx->d_kpt && 2 * (size_t)ctx->n * ctx->L * ctx->K >= need) return CRT_OK;
+    if (!ctx->d_colsum && !dalloc(ctx, &ctx->d_colsum, need)) return CRT_ERR_CUDA;
+    *ws = ctx->d_colsum;
+    return CRT_OK;
 }
 
 template <typename S>
@@ -1904,9 +1910,10 @@ extern "C" int32_t crt_blam0(crt_ctx* ctx, int32_t ldc, int32_t lfpi, double alf
     if ((ldc != 0) != (ctx->sens_real != 0))
         return set_err(ctx, CRT_ERR_ARG, "crt_blam0: ldc does not match the stored Jacobian");
     CK(cudaSetDevice(ctx->device));
-    if (int e = ensure_colsum(ctx)) return e;
-    cd* s = reinterpret_cast<cd*>(ctx->d_colsum);
-    double* jtj = ctx->d_colsum + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
+    double* ws = nullptr;
+    if (int e = colsum_space(ctx, &ws)) return e;
+    cd* s = reinterpret_cast<cd*>(ws);
+    double* jtj = ws + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
     const bool f32 = ctx->prec == CRT_PREC_MIXED;
     if (ldc) {
         if (f32) blam0_launch<float>(ctx, 0, s, jtj);
@@ -1934,8 +1941,9 @@ extern "C" int32_t crt_coverage(crt_ctx* ctx, int32_t part, const double* weight
     if (!ctx->have_sens || !ctx->d_sens) return set_err(ctx, CRT_ERR_ARG, "crt_coverage before crt_jacobian");
     if (!weight && !ctx->d_wd) return set_err(ctx, CRT_ERR_ARG, "crt_coverage without weights before crt_set_data");
     CK(cudaSetDevice(ctx->device));
-    if (int e = ensure_colsum(ctx)) return e;
-    double *w = ctx->d_colsum, *cs = ctx->d_colsum + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
+    double* w = nullptr;
+    if (int e = colsum_space(ctx, &w)) return e;
+    double* cs = w + 2 * (size_t)ctx->N * (1 + BLAM0_SPLIT);
     if (weight) CK(cudaMemcpyAsync(w, weight, sizeof(double) * ctx->N, cudaMemcpyHostToDevice, ctx->st));
     const double* wd = weight ? w : ctx->d_wd;
     const int sq = weight ? 0 : 1, g = (ctx->E * 32 + 255) / 256;

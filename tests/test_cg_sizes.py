@@ -52,3 +52,37 @@ def test_update_where_the_turns_end(nx, nz):
     """24,576 cells, the most that one cluster turns an iteration over for, and
     24,640, by the grid-wide kernels."""
     test_update_and_lambda_candidates(nx, nz, 6, False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ldc", [False, True])
+@pytest.mark.parametrize("nx,nz,nel,spacings,nmax", [(10, 2, 4, (1,), 1), (41, 25, 9, (1, 2), 8), (64, 3, 60, (1, 2), 50)])
+def test_sums_of_a_formed_and_of_a_set_jacobian(nx, nz, nel, spacings, nmax, ldc):
+    """lambda_0 and the coverage, whose sums lie in the Jacobian's workspace
+    where it is long enough: the same from the Jacobian that the context formed
+    and from the same one set on a context without that workspace, and the
+    Jacobian formed again afterwards is unchanged."""
+    from crtomo_stable_b200.lib import Context
+    rng = np.random.default_rng(nx)
+    xs = np.arange(nx + 1, dtype=np.float64) - (nx - nel) // 2
+    mesh = synth.structured_mesh(xs, synth.graded_depths(nz, 0.4, 1.1), triangles=True)
+    enr = synth.surface_electrodes(mesh, xs, np.arange(nel, dtype=np.float64), nz)
+    strnr, vnr = synth.encode(synth.dipole_dipole(nel, spacings, nmax))
+    sigma = synth.sigma_from(rng.uniform(10.0, 1000.0, mesh.elanz), -rng.uniform(1.0, 30.0, mesh.elanz))
+    N = len(strnr)
+    dat, wd, weight = rng.standard_normal(N) + 0j, rng.uniform(0.5, 2.0, N), rng.uniform(0.5, 2.0, N)
+    kw = dict(kwn=np.array([0.05, 0.5]), kwnwi=np.array([0.1, 0.2]))
+    formed, held = Context(mesh, enr, strnr, vnr, **kw), Context(mesh, enr, strnr, vnr, **kw)
+    formed.forward(sigma, ldc=ldc)
+    J = formed.jacobian(mode=1 if ldc else 0)
+    held.set_jacobian(J, real=ldc)
+    out = []
+    for ctx in (formed, held):
+        ctx.set_data(dat, wd)
+        out.append([ctx.blam0(1.0, 1.0, ldc=ldc), ctx.coverage(), ctx.coverage(weight=weight), ctx.blam0(1.0, 1.0, ldc=ldc)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert out[0][0] == out[0][3]
+    assert np.array_equal(formed.jacobian(mode=1 if ldc else 0), J)
+    formed.close()
+    held.close()
